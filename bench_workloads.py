@@ -411,7 +411,7 @@ def run_richards(args, dist, rank, ws, METRIC_NAME):
 
 def run_cholesky(args, dist, rank, ws, METRIC_NAME):
     """The direct solver (linear_solver = cholesky_solver, DPFEHM src/groundwater.jl:56-60): a
-    banded Cholesky factorisation of the FP64 operator on the GPU, for the grid classes the
+    factorisation of the FP64 operator by nested dissection on the GPU, for the grid classes the
     reference's own Cholesky-versus-CG comparison covers (examples/fracture_network_solver_scaling/
     porous_media_comparison.jl: unit conductivity, Dirichlet h = 1 and 0 on the x = min and x = max
     faces). Here: a 2-D grid of 500 x 500 cells and a 3-D grid of 48^3, each with a Matern
@@ -614,7 +614,7 @@ def run(name, args, dist, rank, ws):
     if name == "dfn":
         return run_dfn(args, dist, rank, ws, "forward+adjoint solves/sec, 5M-cell fracture network, CSR path")
     if name == "cholesky":
-        return run_cholesky(args, dist, rank, ws, "forward+adjoint solves/sec, direct (banded Cholesky) solver")
+        return run_cholesky(args, dist, rank, ws, "forward+adjoint solves/sec, direct solver")
     if name == "richards":
         return run_richards(args, dist, rank, ws, "Richards steady forward+adjoint solves/sec, 200k cells")
     if name == "general_1m":

@@ -542,12 +542,12 @@ def amg_solver(*_a, **_k):
 
 def cholesky_solver(*_a, **_k):
     """Selector for ``linear_solver=`` (src/groundwater.jl:56-60): a direct solve. The GPU
-    factors the operator as L L^T in a narrow band (rows renumbered: regular grids with their two
-    shortest axes fastest, other meshes in reverse Cuthill-McKee order) once per assembly and
-    answers each solve with two triangular solves (options ``solver="cholesky"``). A band too wide
-    for the device falls back to the AMG-preconditioned CG run to the FP64 rounding floor of the
-    system (the mixed-precision solver with a tolerance below any floor, whose FP64 check accepts
-    with status OK once the true residual is at the floor)."""
+    factors the operator by nested dissection (dense fronts, level by level) once per assembly
+    and answers each solve with two triangular solves (options ``solver="cholesky"``). A system too
+    large for it (by the half-bandwidth of a narrow band ordering) falls back to the
+    AMG-preconditioned CG run to the FP64 rounding floor of the system (the mixed-precision solver
+    with a tolerance below any floor, whose FP64 check accepts with status OK once the true
+    residual is at the floor)."""
     raise TypeError("cholesky_solver selects the solver; pass it as linear_solver=cholesky_solver")
 
 
@@ -571,7 +571,7 @@ def groundwater_steadystate(Ks, neighbors, areasoverlengths, dirichletnodes, dir
     """Steady-state heads over all cells (src/groundwater.jl:75-83).
 
     ``linear_solver``: ``amg_solver`` (default; CG + AMG to ``reltol``) or ``cholesky_solver``
-    (a banded Cholesky factorisation on the GPU). ``kwargs`` are solver options (reltol, maxiter,
+    (a direct factorisation on the GPU). ``kwargs`` are solver options (reltol, maxiter,
     precision='fp64'|'mixed', solver='cg'|'cholesky', ...).
     """
     N = len(Qs) if not _is_torch(Qs) else Qs.numel()

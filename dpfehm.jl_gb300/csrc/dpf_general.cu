@@ -13,6 +13,7 @@
 #include <numeric>
 
 #include "dpf_direct.h"
+#include "dpf_front.h"
 #include "dpf_general.h"
 #include "dpf_struct_kernels.cuh"
 
@@ -820,6 +821,7 @@ GeneralSolver::GeneralSolver(long long N_, long long F_, const int64_t *a, const
     GCK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev_id));
     long long target = (long long)sms * std::max(1, opt.blocks_per_sm);
     nblocks = (int)std::max(1LL, std::min((N + kBlock - 1) / kBlock, target));
+    if (opt.solver == DPF_SOLVER_CHOLESKY) configure_front_kernels();
     setup_topology(a, b, aol, volumes, nd, dn);
     build_hierarchy();
     // vectors
@@ -1086,12 +1088,15 @@ static unsigned gblocks(long long n, int cap) { return (unsigned)std::max(1LL, s
 void GeneralSolver::assemble(const double *Ks, const double *kc, int kind, const double *shift_, bool init_x) {
     GLevel &L0 = lv[0];
     direct_stale = true;  // a direct factor of the previous operator is out of date
+    choose_direct();
     const int n = (int)N;
     kg_assemble<<<gblocks(n, nblocks), kBlock, 0, stream>>>(n, irp, ifc, fa, fb, faol, Ks, kc, kind, L0.dir, in_dh, in_Q,
                                                            shift_, L0.leak64, b64, h, init_x ? 1 : 0);
     GLAUNCH();
     kg_entry_vals<<<gblocks(L0.nnz, nblocks), kBlock, 0, stream>>>(L0.nnz, e_face, fa, fb, faol, Ks, kc, kind, L0.v64);
     GLAUNCH();
+    GCK(cudaMemsetAsync(d_status, 0, sizeof(int), stream));
+    if (fronts) return;  // the direct solver needs no hierarchy
     for (size_t l = 0; l + 1 < lv.size(); l++) {
         GLevel &Fl = lv[l], &C = lv[l + 1];
         kg_coarse_vals<<<gblocks(C.nnz, nblocks), kBlock, 0, stream>>>(C.nnz, Fl.crp, Fl.cci, Fl.v64, C.v64);
@@ -1115,7 +1120,6 @@ void GeneralSolver::assemble(const double *Ks, const double *kc, int kind, const
         kg_to_df<<<gblocks(n, nblocks), kBlock, 0, stream>>>(n, L0.leak64, leakdf);
         GLAUNCH();
     }
-    GCK(cudaMemsetAsync(d_status, 0, sizeof(int), stream));
     GLevel &Lc = lv.back();
     if (Lc.dense) {
         kg_dense_inverse<<<1, kBlock, 0, stream>>>(Lc.n, Lc.rp, Lc.ci, Lc.v64, Lc.leak64, dense_inv, d_status);
@@ -1289,44 +1293,48 @@ void GeneralSolver::df_pcg(const double *b, double *x, double tol2) {
     }
 }
 
-// The FP64 operator in the banded Cholesky's storage: per row its diagonal leak + the sum of
-// its couplings, and from the row with the smaller index of each coupling -c at (max, min) of the
-// two band rows (added: a pair of cells joined by several faces has several couplings).
-__global__ void kg_band_fill(int n, GOp<double> A, const long long *__restrict__ iperm, long long w,
-                             double *__restrict__ band) {
+// The FP64 operator in the fronts' panels (dpf_front.h): per row its diagonal leak + the sum of its
+// couplings, and from the row with the smaller index of each coupling -c (added: a pair of cells joined
+// by several faces has several couplings).
+__global__ void kg_front_fill(int n, GOp<double> A, const int *__restrict__ iperm, FrontIndex ix) {
     for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < n; i += gridDim.x * blockDim.x) {
-        const long long k = iperm[i];
+        const int k = iperm[i];
         double d = A.leak[i];
         for (int e = A.rp[i]; e < A.rp[i + 1]; e++) {
             const int j = A.ci[e];
+            if (!DPF_INSIDE(CK_CSR_COL, j, 0, n)) continue;
             d += A.v[e];
             if (j > i) {
-                const long long kj = iperm[j];
-                const long long r = max(k, kj), q = min(k, kj);
-                if (r - q <= w) atomicAdd(&band[q * (w + 1) + (r - q)], -A.v[e]);
+                const int kj = iperm[j];
+                double *p = ix.at(max(k, kj), min(k, kj));
+                if (p) atomicAdd(p, -A.v[e]);
             }
         }
-        band[k * (w + 1)] = d;
+        double *p = ix.at(k, k);
+        if (p) *p = d;
     }
 }
 
+// As StructBatch::choose_direct.
+void GeneralSolver::choose_direct() {
+    if (opt.solver != DPF_SOLVER_CHOLESKY || direct_tried) return;
+    direct_tried = true;
+    size_t free_b = 0, total_b = 0;
+    GCK(cudaMemGetInfo(&free_b, &total_b));
+    if (N >= kFrontMaxCells || !direct_fits(N, band_order_rcm(N, hrp_, hci_).w, free_b / 2)) return;
+    fronts = make_fronts(dissect_graph((int)N, hrp_, hci_), hrp_, hci_, free_b / 10 * 9, stream);
+}
+
 bool GeneralSolver::direct_solve(const double *b, double *x) {
+    if (!fronts) return false;
     GLevel &L0 = lv[0];
-    if (!direct_tried) {
-        direct_tried = true;
-        const BandOrder ord = band_order_rcm(N, hrp_, hci_);
-        size_t free_b = 0, total_b = 0;
-        GCK(cudaMemGetInfo(&free_b, &total_b));
-        if (BandCholesky::fits(N, ord.w, free_b / 2)) direct.reset(new BandCholesky(ord, stream));
-    }
-    if (!direct) return false;
-    NvtxRange range("direct solve (banded Cholesky, CSR)");
-    BandCholesky &D = *direct;
+    NvtxRange range("direct solve (CSR)");
+    FrontSolver &D = *fronts;
     D.set_stream(stream);
     const long long l0 = D.launches;
     if (direct_stale) {
         D.clear();
-        kg_band_fill<<<gblocks(N, nblocks), kBlock, 0, stream>>>((int)N, gop<double>(L0), D.iperm(), D.w, D.band());
+        kg_front_fill<<<gblocks(N, nblocks), kBlock, 0, stream>>>((int)N, gop<double>(L0), D.iperm(), D.index());
         GLAUNCH();
         direct_ok = D.factor();
         direct_stale = false;
@@ -1345,10 +1353,9 @@ bool GeneralSolver::direct_solve(const double *b, double *x) {
     D.solve(b, x);
     kg_apply<<<gblocks(N, nblocks), kBlock, 0, stream>>>((int)N, gop<double>(L0), x, r64);
     GLAUNCH();
-    if (!d_direct_acc) d_direct_acc = dev<double>(2);
-    stats_relres = BandCholesky::relres(stream, N, L0.dir, b, r64, d_direct_acc);
+    stats_relres = D.relres(L0.dir, b, r64);
     h_state->status = std::isfinite(stats_relres) ? DPF_OK : DPF_NAN;
-    launches += D.launches - l0 + 2;
+    launches += D.launches - l0;
     return true;
 }
 

@@ -21,6 +21,7 @@
 #include <cooperative_groups.h>
 
 #include "dpf_direct.h"
+#include "dpf_front.h"
 #include "dpf_struct.h"
 #include "dpf_struct_kernels.cuh"
 #include "dpf_plane.cuh"
@@ -1230,18 +1231,19 @@ __global__ void k_apply(const LevelDesc *__restrict__ desc, const int4 *__restri
     }
 }
 
-// The FP64 operator in the banded Cholesky's storage (dpf_direct.h): per cell its diagonal
-// leak + the sum of its face coefficients, and, from the cell on the lower side of each face,
-// the coupling -c at (max, min) of the two cells' band rows. Dirichlet rows are identity rows.
-__global__ void k_band_fill(const LevelDesc *__restrict__ desc, const int4 *__restrict__ bmap, Coeffs<double> C,
-                            const long long *__restrict__ iperm, long long w, double *__restrict__ band) {
+// The FP64 operator in the fronts' panels (dpf_front.h): per cell its diagonal leak + the sum of its
+// face coefficients, and, from the cell on the lower side of each face, the coupling -c. Dirichlet
+// rows are identity rows.
+__global__ void k_front_fill(const LevelDesc *__restrict__ desc, const int4 *__restrict__ bmap, Coeffs<double> C,
+                             const int *__restrict__ iperm, FrontIndex ix) {
     int4 bm = bmap[blockIdx.x];
     const LevelDesc L = desc[bm.x];
     const long long sy = L.nz, sx = (long long)L.ny * L.nz;
     for (int li_ = bm.y * kBlock + (int)threadIdx.x; li_ < (int)L.n; li_ += bm.z * kBlock) {
         Cell c;
         cell_at(L, li_, c);
-        const long long i = c.i, k = iperm[i];
+        const long long i = c.i;
+        const int k = iperm[i];
         double d = C.leak[i];
         const bool up[3] = {c.iz + 1 < L.nz, c.iy + 1 < L.ny, c.ix + 1 < L.nx};
         const long long st[3] = {1, sy, sx};
@@ -1255,12 +1257,13 @@ __global__ void k_band_fill(const LevelDesc *__restrict__ desc, const int4 *__re
             const double v = cf[a][i];
             d += v;
             if (v != 0.0) {
-                const long long kj = iperm[i + st[a]];
-                const long long r = max(k, kj), q = min(k, kj);
-                if (r - q <= w) band[q * (w + 1) + (r - q)] = -v;
+                const int kj = iperm[i + st[a]];
+                double *e = ix.at(max(k, kj), min(k, kj));
+                if (e) *e = -v;
             }
         }
-        band[k * (w + 1)] = d;
+        double *e = ix.at(k, k);
+        if (e) *e = d;
     }
 }
 
@@ -1491,6 +1494,7 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
     }
     // function attributes of this device's kernels, set once before any launch
     configure_kernels();
+    if (opt.solver == DPF_SOLVER_CHOLESKY) configure_front_kernels();
     // launch shape: grids sized to the resident capacity of the device
     int dev = 0, sms = 152;
     CK(cudaGetDevice(&dev));
@@ -1804,6 +1808,7 @@ void StructBatch::write_tail_table() {
 void StructBatch::assemble(const double *Ks, const double *kc, int kind, const double *shift, bool init_x) {
     NvtxRange range("assemble operator and hierarchy");
     direct_stale = true;  // a direct factor of the previous operator is out of date
+    choose_direct();
     Level &L0 = lv[0];
     FaceK fk{Ks, kc, kind};
     if (nb_of(L0.all))
@@ -1816,6 +1821,8 @@ void StructBatch::assemble(const double *Ks, const double *kc, int kind, const d
                 mixed ? cdf[2] : nullptr, mixed ? cdf[3] : nullptr, b64, h, init_x ? 1 : 0);
         }
     LAUNCH_CHECK();
+    have_operator = true;
+    if (fronts) return;  // the direct solver needs no hierarchy
     for (int l = 0; l + 1 < nlev_max; l++) {
         Level &F = lv[l], &C = lv[l + 1];
         if (!nb_of(C.all)) continue;
@@ -1850,7 +1857,6 @@ void StructBatch::assemble(const double *Ks, const double *kc, int kind, const d
         }
         LAUNCH_CHECK();
     }
-    have_operator = true;
 }
 
 // ---- V-cycle: z = M r on the fine level (vector precision T)
@@ -2775,31 +2781,39 @@ void StructBatch::apply(const double *x, double *y) {
     LAUNCH_CHECK();
 }
 
-bool StructBatch::direct_solve(const double *b, double *x) {
+// Chooses the solver of a handle that asks for the direct one: the fronts when the system is within
+// direct_fits' limit and they fit the device, else none (the iterative solver runs). Before the first
+// assembly, which then leaves out the multigrid hierarchy that only the iterative solver needs.
+void StructBatch::choose_direct() {
+    if (opt.solver != DPF_SOLVER_CHOLESKY || direct_tried) return;
+    direct_tried = true;
     Level &L0 = lv[0];
-    if (!direct_tried) {
-        direct_tried = true;
-        std::vector<std::array<int, 3>> dims;
-        std::vector<long long> off;
-        for (int p = 0; p < nprob; p++) {
-            const LevelDesc &D = L0.h_desc[p];
-            dims.push_back({D.nx, D.ny, D.nz});
-            off.push_back(D.off);
-        }
-        const BandOrder ord = band_order_regular(dims, off);
-        size_t free_b = 0, total_b = 0;
-        CK(cudaMemGetInfo(&free_b, &total_b));
-        if (BandCholesky::fits(N, ord.w, free_b / 2)) direct.reset(new BandCholesky(ord, stream));
+    std::vector<std::array<int, 3>> dims;
+    std::vector<long long> off;
+    for (int p = 0; p < nprob; p++) {
+        const LevelDesc &D = L0.h_desc[p];
+        dims.push_back({D.nx, D.ny, D.nz});
+        off.push_back(D.off);
     }
-    if (!direct) return false;
-    NvtxRange range("direct solve (banded Cholesky)");
-    BandCholesky &D = *direct;
+    size_t free_b = 0, total_b = 0;
+    CK(cudaMemGetInfo(&free_b, &total_b));
+    if (N >= kFrontMaxCells || !direct_fits(N, band_order_regular(dims, off).w, free_b / 2)) return;
+    std::vector<int> rp, ci;
+    regular_graph(dims, off, rp, ci);
+    fronts = make_fronts(dissect_regular(dims, off), rp, ci, free_b / 10 * 9, stream);
+}
+
+bool StructBatch::direct_solve(const double *b, double *x) {
+    if (!fronts) return false;
+    Level &L0 = lv[0];
+    NvtxRange range("direct solve");
+    FrontSolver &D = *fronts;
     D.set_stream(stream);
     const long long l0 = D.launches;
     if (direct_stale) {
         D.clear();
-        k_band_fill<<<nb_of(L0.all), kBlock, 0, stream>>>(L0.d_desc, L0.all.d_map, coeffs_of<double>(L0, true),
-                                                         D.iperm(), D.w, D.band());
+        k_front_fill<<<nb_of(L0.all), kBlock, 0, stream>>>(L0.d_desc, L0.all.d_map, coeffs_of<double>(L0, true),
+                                                          D.iperm(), D.index());
         LAUNCH_CHECK();
         direct_ok = D.factor();
         direct_stale = false;
@@ -2816,11 +2830,10 @@ bool StructBatch::direct_solve(const double *b, double *x) {
     D.solve(b, x);
     // the relative residual over the free cells, for the statistics
     apply(x, r64);
-    if (!d_direct_acc) d_direct_acc = (double *)dalloc_bytes(2 * sizeof(double));
-    stats_relres = BandCholesky::relres(stream, N, L0.dir, b, r64, d_direct_acc);
+    stats_relres = D.relres(L0.dir, b, r64);
     last_status = std::isfinite(stats_relres) ? DPF_OK : DPF_NAN;
     if (last_status != DPF_OK) last_message = "non-finite residual after the direct solve";
-    launches += D.launches - l0 + 2;
+    launches += D.launches - l0;
     return true;
 }
 

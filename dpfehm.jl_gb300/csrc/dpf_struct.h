@@ -35,7 +35,7 @@ struct GridSpec {
 };
 
 class StructBatch;
-class BandCholesky;
+class FrontSolver;
 
 // Counts every kernel launch and, while profiling is on, brackets it with a pair
 // of CUDA events on the launching stream (per-kernel device time).
@@ -141,13 +141,12 @@ public:
     template <typename T>
     void pcg_iteration(T *x);
     void df_iteration(double *x64);
-    // options.solver = DPF_SOLVER_CHOLESKY: x = A^-1 b by the banded Cholesky factor of the FP64
-    // operator (factored again after each assembly); false when the band is too wide for the device
-    // (the iterative solve then runs instead)
+    // options.solver = DPF_SOLVER_CHOLESKY: x = A^-1 b by a factor of the FP64 operator (factored again
+    // after each assembly); false when the system is too large for it (the iterative solve then runs)
     bool direct_solve(const double *b, double *x);
-    std::unique_ptr<BandCholesky> direct;
+    void choose_direct();
+    std::unique_ptr<FrontSolver> fronts;
     bool direct_tried = false, direct_stale = true, direct_ok = false;
-    double *d_direct_acc = nullptr;  // the direct solve's residual sums
     cudaGraphExec_t loop_graph(int kind, void *x);
     void run_loop(int kind, void *x);
     int read_count(int which);

@@ -128,8 +128,8 @@ function adjoint(p::Problem, delta)
 end
 
 """Selectors for the `linear_solver` keyword: `amg_solver` (CG + AMG to reltol, the default)
-and `cholesky_solver` (a banded Cholesky factorisation of the operator on the GPU; a band too
-wide for the device falls back to the CG solver run to the FP64 rounding floor)."""
+and `cholesky_solver` (a direct factorisation of the operator on the GPU; a system too
+large for it falls back to the CG solver run to the FP64 rounding floor)."""
 function amg_solver end
 function cholesky_solver end
 

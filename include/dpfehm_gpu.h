@@ -68,12 +68,13 @@ typedef enum {
 
 typedef enum {
     DPF_SOLVER_CG = 0,       /* AMG-preconditioned CG to reltol (the reference's amg_solver) */
-    DPF_SOLVER_CHOLESKY = 1  /* banded Cholesky factorisation of the FP64 operator (the reference's
-                                cholesky_solver, src/groundwater.jl:56-60): the rows renumbered into a
-                                narrow band (regular grids: the two shortest axes fastest; other meshes:
-                                reverse Cuthill-McKee), factored once per assembly, two triangular solves
-                                per solve; a band too wide for the device (more than half its free memory,
-                                or above about 2e13 multiply-adds) falls back to the CG solve */
+    DPF_SOLVER_CHOLESKY = 1  /* direct factorisation of the FP64 operator (the reference's
+                                cholesky_solver, src/groundwater.jl:56-60): nested dissection and dense
+                                fronts, factored once per assembly, two triangular solves per solve. Taken
+                                for systems whose narrow band ordering (regular grids: the two shortest
+                                axes fastest; other meshes: reverse Cuthill-McKee) has a half-bandwidth w
+                                with n (w + 1) doubles within half the device's free memory and n w^2 up
+                                to 2e13; larger ones fall back to the CG solve */
 } dpf_solver;
 
 typedef struct dpf_options {
@@ -372,7 +373,7 @@ int dpf_debug_expired_wait(double *waited_ms);
  * (outputs then unspecified). All outputs are device arrays of n entries. */
 int dpf_debug_split48(int64_t n, const double *v, float *hi, float *lo, double *v48, int *ok);
 
-/* No counterpart in the reference. The band orderings of the direct solver, run on the host (no
+/* No counterpart in the reference. The band orderings that size the direct solver, run on the host (no
  * device needed): for a symmetric graph in CSR form (rp[n + 1], ci, host arrays) the reverse
  * Cuthill-McKee order; for nprob regular grids (dims[3 p .. 3 p + 2] = nx, ny, nz, cells z fastest,
  * problems one after another) the order with each grid's two shortest axes fastest. perm[k] (n
