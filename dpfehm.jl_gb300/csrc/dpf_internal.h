@@ -113,6 +113,7 @@ template <typename T>
 struct Coeffs {
     const coef_t<T> *cx, *cy, *cz, *leak;
     const T *idg;                  // inverse diagonal
+    const T *dg;                   // FP64 levels: the diagonal (null on FP32 levels)
 };
 
 // Per-level pointers and the Chebyshev parameters of the fused small-level tail kernel.

@@ -237,16 +237,22 @@ __device__ __forceinline__ T ldv(const T *p, long long i) {
     else return p[i];
 }
 
-// first Chebyshev step from a zero guess: x = d = invtheta D^-1 b
+// first Chebyshev step from a zero guess: x = d = invtheta D^-1 b. FP64 levels keep the direction as
+// e = D d: the step is then x + D^-1 e with e = c1 e + c2 r, one FP64 instruction less per cell than
+// scaling each residual
 template <typename T, bool CG = false>
 __device__ __forceinline__ void cell_cheb_first(const LevelDesc &L, const Cell &c, const Coeffs<T> &C,
                                                 const T *__restrict__ b, T *__restrict__ x, T *__restrict__ d,
                                                 T invtheta) {
-    T v;
-    if constexpr (sizeof(T) == 8) v = invtheta * ldv<CG>(b, c.i) * C.idg[c.i];
-    else v = invtheta * __fdividef(ldv<CG>(b, c.i), diag7(L, c, C));
-    x[c.i] = v;
-    d[c.i] = v;
+    if constexpr (sizeof(T) == 8) {
+        const T e = invtheta * ldv<CG>(b, c.i);
+        x[c.i] = e * C.idg[c.i];
+        d[c.i] = e;
+    } else {
+        const T v = invtheta * __fdividef(ldv<CG>(b, c.i), diag7(L, c, C));
+        x[c.i] = v;
+        d[c.i] = v;
+    }
 }
 
 // the first two Chebyshev steps from a zero guess (see k_cheb_first2)
@@ -256,12 +262,21 @@ __device__ __forceinline__ void cell_cheb_first2(const LevelDesc &L, const Cell 
                                                  T invtheta, T c1, T c2) {
     const T *__restrict__ g = C.idg;
     const T bi = ldv<CG>(b, c.i), gi = g[c.i];
-    const T x1 = invtheta * bi * gi;
-    T Ax, dg;
-    apply7(L, c, C, x1, [&](long long j, int, int, int) { return invtheta * ldv<CG>(b, j) * g[j]; }, Ax, dg);
-    const T dn = c1 * x1 + c2 * (bi - Ax) * gi;
-    d[c.i] = dn;
-    xout[c.i] = x1 + dn;
+    T dg;
+    if constexpr (sizeof(T) == 8) {
+        const T u = bi * gi;  // x1 = invtheta u
+        const T t = resid7(L, c, C, T(0), u, [&](long long j, int, int, int) { return ldv<CG>(b, j) * g[j]; }, dg);
+        const T e = fma(c2, fma(invtheta, t, bi), c1 * invtheta * bi);
+        d[c.i] = e;
+        xout[c.i] = fma(gi, e, invtheta * u);
+    } else {
+        const T x1 = invtheta * bi * gi;
+        const T r = resid7(L, c, C, bi, x1, [&](long long j, int, int, int) { return invtheta * ldv<CG>(b, j) * g[j]; },
+                           dg);
+        const T dn = c1 * x1 + c2 * r * gi;
+        d[c.i] = dn;
+        xout[c.i] = x1 + dn;
+    }
 }
 
 // one Chebyshev step (see k_cheb_step); returns the new iterate
@@ -269,12 +284,18 @@ template <typename T, bool FIRST, bool CG = false>
 __device__ __forceinline__ T cell_cheb_step(const LevelDesc &L, const Cell &c, const Coeffs<T> &C,
                                             const T *__restrict__ b, const T *__restrict__ xin,
                                             T *__restrict__ xout, T *__restrict__ d, T c1, T c2, T &bi) {
-    T xi = ldv<CG>(xin, c.i), Ax, dg;
-    apply7(L, c, C, xi, [&](long long j, int, int, int) { return ldv<CG>(xin, j); }, Ax, dg);
+    T xi = ldv<CG>(xin, c.i), dg;
     bi = ldv<CG>(b, c.i);
-    T r = dinv_times(C, c.i, bi - Ax, dg);
-    T dn = FIRST ? c2 * r : c1 * ldv<CG>((const T *)d, c.i) + c2 * r;
-    T xo = xi + dn;
+    const T ri = resid7(L, c, C, bi, xi, [&](long long j, int, int, int) { return ldv<CG>(xin, j); }, dg);
+    T dn, xo;
+    if constexpr (sizeof(T) == 8) {
+        dn = FIRST ? c2 * ri : fma(c2, ri, c1 * ldv<CG>((const T *)d, c.i));
+        xo = fma(C.idg[c.i], dn, xi);
+    } else {
+        const T r = dinv_times(C, c.i, ri, dg);
+        dn = FIRST ? c2 * r : c1 * ldv<CG>((const T *)d, c.i) + c2 * r;
+        xo = xi + dn;
+    }
     d[c.i] = dn;
     xout[c.i] = xo;
     return xo;
@@ -294,9 +315,9 @@ __device__ __forceinline__ T cell_restrict(const LevelDesc &L, const Cell &cc, c
                 Cell c;
                 c.ix = fx; c.iy = fy; c.iz = fz;
                 c.i = L.off + fx * fsx + fy * fsy + fz;
-                T xi = ldv<CG>(x, c.i), Ax, dg;
-                apply7(L, c, C, xi, [&](long long j, int, int, int) { return ldv<CG>(x, j); }, Ax, dg);
-                acc += ldv<CG>(b, c.i) - Ax;
+                T xi = ldv<CG>(x, c.i), dg;
+                acc += resid7(L, c, C, ldv<CG>(b, c.i), xi, [&](long long j, int, int, int) { return ldv<CG>(x, j); },
+                              dg);
             }
     return acc;
 }
@@ -453,32 +474,16 @@ __global__ void k_coarse_solve(const LevelDesc *__restrict__ desc, const int *__
 // and the same result as the per-level kernels: the corrected iterate of level lt
 // lands in its xb buffer.
 
-template <typename T, bool CLUSTER>
-__global__ void __launch_bounds__(kTailThreads) k_tail_cycle(const TailLevel<T> *__restrict__ tl,
-                                                             const int4 *__restrict__ tails, const CgState *st,
-                                                             const double *__restrict__ Inv, TailParams<T> tp) {
-    pdl_enter();
-    // one problem per block, or (CLUSTER) per thread-block cluster: its blocks share every
-    // step's cells and meet at hardware cluster barriers
-    unsigned rank = 0, nranks = 1;
-    if constexpr (CLUSTER) {
-        rank = cg::this_cluster().block_rank();
-        nranks = cg::this_cluster().num_blocks();
-    }
-    const int4 t = tails[blockIdx.x / nranks];  // problem, first tail level, coarsest level
-    const int p = t.x, lt = t.y, lc = t.z;
-    if (st && !st[p].active) return;  // uniform over the problem's blocks
-    auto sync = [&]() {
-        if constexpr (CLUSTER) cg::this_cluster().sync();
-        else __syncthreads();
-    };
-    const int first = (int)(rank * blockDim.x + threadIdx.x);
-    const int stride = (int)(nranks * blockDim.x);
+// One problem's V-cycle from level lt down to its coarsest level lc and back, by `stride` threads with
+// the barrier `sync` between steps; the corrected iterate of level lt lands in its xb buffer.
+template <typename T, bool CLUSTER, typename Lev, typename Desc, typename Sync>
+__device__ __forceinline__ void tail_cycle(Lev level, Desc descof, int lt, int lc, const double *Ip,
+                                           const TailParams<T> &tp, unsigned rank, int first, int stride, Sync sync) {
     const int deg = tp.deg;
     // descend
     for (int l = lt; l < lc; l++) {
-        const TailLevel<T> V = tl[l];
-        const LevelDesc L = V.desc[p];
+        const TailLevel<T> V = level(l);
+        const LevelDesc L = descof(l);
         T *cur = V.xa, *oth = V.xb;
         int k0 = 1;
         if (deg >= 2) {
@@ -508,8 +513,8 @@ __global__ void __launch_bounds__(kTailThreads) k_tail_cycle(const TailLevel<T> 
             sync();
             T *tmp = cur; cur = oth; oth = tmp;
         }
-        const TailLevel<T> W = tl[l + 1];
-        const LevelDesc Lc = W.desc[p];
+        const TailLevel<T> W = level(l + 1);
+        const LevelDesc Lc = descof(l + 1);
         for (int li = first; li < (int)Lc.n; li += stride) {
             Cell cc;
             cell_at(Lc, li, cc);
@@ -519,23 +524,27 @@ __global__ void __launch_bounds__(kTailThreads) k_tail_cycle(const TailLevel<T> 
     }
     // coarsest: x = A^-1 b with the stored dense inverse (first block of the problem)
     {
-        const TailLevel<T> V = tl[lc];
-        const LevelDesc L = V.desc[p];
-        const double *Ip = Inv + (long long)p * kMaxCoarse * kMaxCoarse;
-        const int i = threadIdx.x;
-        if (rank == 0 && i < (int)L.n) {
+        const TailLevel<T> V = level(lc);
+        const LevelDesc L = descof(lc);
+        // eight lanes per row: a row's products in one chain took longer than the level's smoothing
+        if (rank == 0 && threadIdx.x < 8 * kMaxCoarse) {
+            const int i = threadIdx.x >> 3, s = threadIdx.x & 7;
             double xi = 0.0;
-            for (int j = 0; j < (int)L.n; j++) xi += Ip[j * kMaxCoarse + i] * (double)ldv<CLUSTER>(V.b, L.off + j);
-            V.xb[L.off + i] = (T)xi;
+            if (i < (int)L.n)
+                for (int j = s; j < (int)L.n; j += 8)
+                    xi = fma(Ip[j * kMaxCoarse + i], (double)ldv<CLUSTER>(V.b, L.off + j), xi);
+#pragma unroll
+            for (int o = 4; o > 0; o >>= 1) xi += __shfl_xor_sync(0xffffffffu, xi, o);
+            if (i < (int)L.n && s == 0) V.xb[L.off + i] = (T)xi;
         }
         sync();
     }
     // ascend: prolongation in place into the pre-smoothed iterate, then deg steps
     for (int l = lc - 1; l >= lt; l--) {
-        const TailLevel<T> V = tl[l];
-        const LevelDesc L = V.desc[p];
-        const TailLevel<T> W = tl[l + 1];
-        const LevelDesc Lc = W.desc[p];
+        const TailLevel<T> V = level(l);
+        const LevelDesc L = descof(l);
+        const TailLevel<T> W = level(l + 1);
+        const LevelDesc Lc = descof(l + 1);
         T *cur = (deg % 2 == 0) ? V.xb : V.xa;  // where pre-smoothing left its iterate
         for (int li = first; li < (int)L.n; li += stride) {
             Cell c;
@@ -558,6 +567,28 @@ __global__ void __launch_bounds__(kTailThreads) k_tail_cycle(const TailLevel<T> 
             cur = o;
         }
     }
+}
+
+template <typename T, bool CLUSTER>
+__global__ void __launch_bounds__(kTailThreads) k_tail_cycle(const TailLevel<T> *__restrict__ tl,
+                                                             const int4 *__restrict__ tails, const CgState *st,
+                                                             const double *__restrict__ Inv, TailParams<T> tp) {
+    pdl_enter();
+    // one problem per block, or (CLUSTER) per thread-block cluster: its blocks share every
+    // step's cells and meet at hardware cluster barriers
+    unsigned rank = 0, nranks = 1;
+    if constexpr (CLUSTER) {
+        rank = cg::this_cluster().block_rank();
+        nranks = cg::this_cluster().num_blocks();
+    }
+    const int4 t = tails[blockIdx.x / nranks];  // problem, first tail level, coarsest level
+    if (st && !st[t.x].active) return;          // uniform over the problem's blocks
+    tail_cycle<T, CLUSTER>([&](int l) { return tl[l]; }, [&](int l) { return tl[l].desc[t.x]; }, t.y, t.z,
+                           Inv + (long long)t.x * kMaxCoarse * kMaxCoarse, tp, rank, (int)(rank * blockDim.x + threadIdx.x),
+                           (int)(nranks * blockDim.x), [] {
+                               if constexpr (CLUSTER) cg::this_cluster().sync();
+                               else __syncthreads();
+                           });
 }
 
 // ---------------------------------------------------------------- CG kernels
@@ -688,6 +719,20 @@ __global__ void k_update_p(const LevelDesc *__restrict__ desc, const int4 *__res
 // on the true FP64 residual, and another round runs if it is not met.
 
 
+// (A p)_i in double-float, flux form, p at the cell and its neighbours
+__device__ __forceinline__ float2 cell_df_apply(const LevelDesc &L, const Cell &c, const CoeffsDF &C, float2 pi,
+                                                const float2 *pv) {
+    const long long i = c.i, sy = L.nz, sx = (long long)L.ny * L.nz;
+    float2 a = df_mul(C.leak[i], pi);
+    if (c.iz + 1 < L.nz) a = df_add(a, df_mul(C.cz[i], df_sub(pi, pv[i + 1])));
+    if (c.iz > 0) a = df_add(a, df_mul(C.cz[i - 1], df_sub(pi, pv[i - 1])));
+    if (c.iy + 1 < L.ny) a = df_add(a, df_mul(C.cy[i], df_sub(pi, pv[i + sy])));
+    if (c.iy > 0) a = df_add(a, df_mul(C.cy[i - sy], df_sub(pi, pv[i - sy])));
+    if (c.ix + 1 < L.nx) a = df_add(a, df_mul(C.cx[i], df_sub(pi, pv[i + sx])));
+    if (c.ix > 0) a = df_add(a, df_mul(C.cx[i - sx], df_sub(pi, pv[i - sx])));
+    return a;
+}
+
 // q = A p in double-float (flux form); alpha = rz / (p . q) (hi parts: q is accurate, so
 // its leading float is too)
 #ifndef DPF_DF_SPMV_MINB
@@ -699,20 +744,12 @@ __global__ void __launch_bounds__(kBlock, DPF_DF_SPMV_MINB) k_df_spmv_pq(const L
     pdl_enter();
     DPF_BLOCK_PROLOGUE(desc, bmap, st)
     Acc<float> part;
-    const long long sy = L.nz, sx = (long long)L.ny * L.nz;
     for (int li_ = bm.y * kBlock + (int)threadIdx.x; li_ < (int)L.n; li_ += bm.z * kBlock) {
         Cell c;
         cell_at(L, li_, c);
-        const long long i = c.i;
-        const float2 pi = pv[i];
-        float2 a = df_mul(C.leak[i], pi);
-        if (c.iz + 1 < L.nz) a = df_add(a, df_mul(C.cz[i], df_sub(pi, pv[i + 1])));
-        if (c.iz > 0) a = df_add(a, df_mul(C.cz[i - 1], df_sub(pi, pv[i - 1])));
-        if (c.iy + 1 < L.ny) a = df_add(a, df_mul(C.cy[i], df_sub(pi, pv[i + sy])));
-        if (c.iy > 0) a = df_add(a, df_mul(C.cy[i - sy], df_sub(pi, pv[i - sy])));
-        if (c.ix + 1 < L.nx) a = df_add(a, df_mul(C.cx[i], df_sub(pi, pv[i + sx])));
-        if (c.ix > 0) a = df_add(a, df_mul(C.cx[i - sx], df_sub(pi, pv[i - sx])));
-        q[i] = a;
+        const float2 pi = pv[c.i];
+        const float2 a = cell_df_apply(L, c, C, pi, pv);
+        q[c.i] = a;
         part = part + Acc<float>::prod(pi.x, a.x);
     }
     double2 tot;
@@ -768,6 +805,55 @@ __global__ void k_df_update_p(const LevelDesc *__restrict__ desc, const int4 *__
     }
 }
 
+// The outcome of a true-residual check (totals: |r|^2 and |b|^2 at the start, |r|^2 and the rounding floor
+// after a round): whether the problem takes part in a (further) round.
+__device__ __forceinline__ void check_round(CgState &s, bool first, double2 tot, double tol2, int maxiter,
+                                            int max_rounds, int *active_count) {
+    s.orr = tot.x;
+    bool go;
+    if (first) {
+        s.floor2 = 0.0;
+        s.obb = tot.y;
+        s.tol2 = tol2;
+        s.status = DPF_OK;
+        s.total_iters = 0;
+        s.outer = 0;
+        s.stall = 0;
+        go = s.obb > 0.0 && s.orr > tol2 * s.obb;
+        if (!isfinite(s.orr)) { s.status = DPF_NAN; go = false; }
+    } else {
+        s.outer++;
+        s.floor2 = tot.y;
+        // the true residual is at the FP64 rounding floor of b - A x when it is within the
+        // floor's bound, or when a whole round did not even halve it: no further accuracy
+        // exists in FP64, so the solve is accepted there
+        const bool at_floor = s.orr <= s.floor2 || s.orr > 0.25 * s.orr_prev;
+        go = true;
+        if (!isfinite(s.orr)) { s.status = DPF_NAN; go = false; }
+        else if (s.orr <= tol2 * s.obb || at_floor) go = false;
+        else if (s.total_iters >= maxiter || s.outer >= max_rounds) { s.status = DPF_NOT_CONVERGED; go = false; }
+    }
+    s.orr_prev = s.orr;
+    s.ru_flag = go ? 1 : 0;  // problem takes part in the next round
+    s.active = go ? 1 : 0;
+    if (first) {
+        s.iters = 0;
+        s.rz = 0.0;
+        s.rz_old = 0.0;
+        s.beta = 0.0;
+        s.cont = 1.0;
+    }
+    if (go) {
+        // a further round continues the Krylov process on the true residual (residual
+        // replacement): the direction is kept, and the next beta is rescaled by the change
+        // of normalisation new/old so that p = z + beta p holds in the new units
+        const double sc = sqrt(s.orr);
+        if (!first) s.cont = sc / s.scale;
+        s.scale = sc;
+        atomicAdd(active_count, 1);
+    }
+}
+
 // True residual r64 = b - A x64 in FP64 flux form; decides whether a (further) round is
 // needed. FIRST: the start of a solve. ZERO (with FIRST): the initial guess is zero on
 // free cells and the Dirichlet value on identity rows, so r = b on free rows and 0 on
@@ -820,50 +906,7 @@ __global__ void k_df_residual(const LevelDesc *__restrict__ desc, const int4 *__
     if (!FIRST) bb.v *= 0x1p-96;
     double2 tot;
     if (reduce_last<double, 2>(rr, bb, rs, pinfo[p], p, tot) && threadIdx.x == 0) {
-        CgState &s = st[p];
-        s.orr = tot.x;
-        bool go;
-        if (FIRST) {
-            s.floor2 = 0.0;
-            s.obb = tot.y;
-            s.tol2 = tol2;
-            s.status = DPF_OK;
-            s.total_iters = 0;
-            s.outer = 0;
-            s.stall = 0;
-            go = s.obb > 0.0 && s.orr > tol2 * s.obb;
-            if (!isfinite(s.orr)) { s.status = DPF_NAN; go = false; }
-        } else {
-            s.outer++;
-            s.floor2 = tot.y;
-            // the true residual is at the FP64 rounding floor of b - A x when it is within the
-            // floor's bound, or when a whole round did not even halve it: no further accuracy
-            // exists in FP64, so the solve is accepted there
-            const bool at_floor = s.orr <= s.floor2 || s.orr > 0.25 * s.orr_prev;
-            go = true;
-            if (!isfinite(s.orr)) { s.status = DPF_NAN; go = false; }
-            else if (s.orr <= tol2 * s.obb || at_floor) go = false;
-            else if (s.total_iters >= maxiter || s.outer >= max_rounds) { s.status = DPF_NOT_CONVERGED; go = false; }
-        }
-        s.orr_prev = s.orr;
-        s.ru_flag = go ? 1 : 0;  // problem takes part in the next round
-        s.active = go ? 1 : 0;
-        if (FIRST) {
-            s.iters = 0;
-            s.rz = 0.0;
-            s.rz_old = 0.0;
-            s.beta = 0.0;
-            s.cont = 1.0;
-        }
-        if (go) {
-            // a further round continues the Krylov process on the true residual (residual
-            // replacement): the direction is kept, and the next beta is rescaled by the change
-            // of normalisation new/old so that p = z + beta p holds in the new units
-            const double sc = sqrt(s.orr);
-            if (!FIRST) s.cont = sc / s.scale;
-            s.scale = sc;
-            atomicAdd(active_count, 1);
-        }
+        check_round(st[p], FIRST, tot, tol2, maxiter, max_rounds, active_count);
     }
 }
 
@@ -1105,10 +1148,11 @@ __global__ void k_cell_k(const LevelDesc *__restrict__ desc, const int4 *__restr
     }
 }
 
-// inverse diagonal of a level from its FP64 coefficients (the smoothers multiply
-// instead of dividing); written in FP64 and/or FP32
+// the smoothers' diagonals of a level: FP64 levels the diagonal and its inverse (they multiply
+// instead of dividing), FP32 levels the inverse
 __global__ void k_invdiag(const LevelDesc *__restrict__ desc, const int4 *__restrict__ bmap, Coeffs<double> C,
-                          Coeffs<float> C16, double *__restrict__ idg, float *__restrict__ idg32) {
+                          Coeffs<float> C16, double *__restrict__ idg, double *__restrict__ dg,
+                          float *__restrict__ idg32) {
     pdl_enter();
     int4 bm = bmap[blockIdx.x];
     const LevelDesc L = desc[bm.x];
@@ -1116,9 +1160,9 @@ __global__ void k_invdiag(const LevelDesc *__restrict__ desc, const int4 *__rest
         Cell c;
         cell_at(L, li_, c);
         if (idg) {
-            const double v = 1.0 / diag7(L, c, C);
-            idg[c.i] = v;
-            if (idg32) idg32[c.i] = (float)v;
+            const double v = diag7(L, c, C);
+            dg[c.i] = v;
+            idg[c.i] = 1.0 / v;
         } else {
             // the FP32 V-cycle: the diagonal its kernels form from the bf16 coefficients
             idg32[c.i] = 1.0f / diag7(L, c, C16);
@@ -1267,6 +1311,10 @@ __global__ void k_front_fill(const LevelDesc *__restrict__ desc, const int4 *__r
     }
 }
 
+}  // namespace dpf
+#include "dpf_persist.cuh"
+namespace dpf {
+
 // ================================================================ host side
 static void ck(cudaError_t e, const char *what) {
     if (e != cudaSuccess) throw CudaError(std::string(what) + ": " + cudaGetErrorString(e), e);
@@ -1334,6 +1382,8 @@ static void check_fast_div(unsigned d, unsigned m, int l, unsigned nmax) {
     for (unsigned n = 0; n < nmax && n < 4096; n++)
         if (q(n) != n / d) throw DpfError("invariant-integer division self-check failed", DPF_CUDA);
 }
+
+constexpr int kCountWords = 32 + kGridBarWords;
 
 // Launch map over the problems marked in `take`. Kernels loop over their cells with a
 // stride of (blocks of the problem) x kBlock, so a problem's block count is chosen to
@@ -1463,6 +1513,51 @@ void StructBatch::build_plane_items(PlaneItems &P, const Level &L, const std::ve
     P.ok = true;
 }
 
+// The shares of a level for the persistent kernel: at most one per block, so that a step is one pass over
+// equal numbers of cells, at least 32 each. Problems of one size get the same number (their sums
+// then group alike); blocks left over go to the size with the largest shares.
+void StructBatch::build_pieces(Pieces &P, const std::vector<LevelDesc> &desc, const std::vector<int> &take) {
+    long long total = 0, taken = 0;
+    std::map<long long, int> sizes;  // cells -> problems
+    for (int p = 0; p < nprob; p++)
+        if (take[p]) {
+            taken++;
+            total += desc[p].n;
+            sizes[desc[p].n]++;
+        }
+    std::map<long long, long long> share;  // cells -> shares per problem
+    long long used = 0;
+    auto most = [](long long n) { return (n + 31) / 32; };
+    for (auto &s : sizes) {
+        share[s.first] = std::min(most(s.first), 1 + (long long)((double)(persist_blocks - taken) * s.first / total));
+        used += share[s.first] * s.second;
+    }
+    for (;;) {
+        long long best = 0;
+        for (auto &s : sizes)
+            if (used + s.second <= persist_blocks && share[s.first] < most(s.first) &&
+                (!best || s.first * share[best] > best * share[s.first]))
+                best = s.first;
+        if (!best) break;
+        share[best]++;
+        used += sizes[best];
+    }
+    std::vector<int4> list;
+    std::vector<int2> pinfo(nprob, make_int2(0, 0));
+    for (int p = 0; p < nprob; p++) {
+        if (!take[p]) continue;
+        const int k = (int)share[desc[p].n];
+        pinfo[p] = make_int2((int)list.size(), k);
+        for (int q = 0; q < k; q++) list.push_back(make_int4(p, q, k, 0));
+    }
+    P.n = (int)list.size();
+    if (nprob == 1) return;  // the kernel works a single problem's shares out itself
+    P.list = dalloc<int4>(list.size(), owned);
+    P.pinfo = dalloc<int2>(nprob, owned);
+    if (!list.empty()) CK(cudaMemcpy(P.list, list.data(), list.size() * sizeof(int4), cudaMemcpyHostToDevice));
+    CK(cudaMemcpy(P.pinfo, pinfo.data(), nprob * sizeof(int2), cudaMemcpyHostToDevice));
+}
+
 StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<std::vector<int64_t>> &dnodes,
                          const dpf_options &o, cudaStream_t s)
     : opt(o), stream(s) {
@@ -1500,6 +1595,17 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
     CK(cudaGetDevice(&dev));
     CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
     const long long target_blocks = (long long)sms * std::max(1, opt.blocks_per_sm);
+    // the persistent solve: one block per SM, all resident
+    {
+        int coop = 0, occ = 0;
+        CK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev));
+        const void *k = mixed ? (nprob == 1 ? (const void *)k_solve_persistent<float, true>
+                                            : (const void *)k_solve_persistent<float, false>)
+                              : (nprob == 1 ? (const void *)k_solve_persistent<double, true>
+                                            : (const void *)k_solve_persistent<double, false>);
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kPersistThreads, 0));
+        if (coop && occ >= 1 && nlev_max <= kPersistLevels && nprob <= std::min(sms, kPersistProblems)) persist_blocks = sms;
+    }
     // fused tail: from the first level (>= 1) at which a problem has at most tail_cells cells
     std::vector<int> tail_at(nprob);
     for (int p = 0; p < nprob; p++) {
@@ -1510,6 +1616,16 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
             if ((long long)d[0] * d[1] * d[2] <= opt.tail_cells) { tail_at[p] = l; break; }
         }
         if (tail_at[p] < nlev[p]) tails.push_back(make_int4(p, tail_at[p], nlev[p] - 1, 0));
+    }
+    // the persistent kernel's own tail: one block per problem from the first level (>= 1) small enough
+    // that its steps cost less there than at grid barriers (about 3 us a step): FP64 steps are bound by
+    // one SM's FP64 pipe already at a few hundred cells
+    std::vector<int> ptail(nprob);
+    for (int p = 0; p < nprob; p++) {
+        ptail[p] = nlev[p] - 1;
+        for (int l = nlev[p] - 1; l >= 1; l--)
+            if ((long long)shapes[p][l][0] * shapes[p][l][1] * shapes[p][l][2] <= (mixed ? kPersistTail32 : kPersistTail64))
+                ptail[p] = l;
     }
     // level descriptors
     lv.resize(nlev_max);
@@ -1563,6 +1679,16 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
         if (l == 0)
             build_plane_items(L.pa, L, has, sms, opt.df_plane_cells > 0 ? kPlaneThreads : 0, opt.df_plane_blocks_per_sm,
                               nullptr, l);
+        if (persist_blocks) {
+            std::vector<int> psm(nprob, 0), pre(nprob, 0);
+            for (int p = 0; p < nprob; p++) {
+                psm[p] = l < ptail[p];
+                pre[p] = l >= 1 && l <= ptail[p];
+            }
+            if (l == 0) build_pieces(pall, L.h_desc, has);
+            build_pieces(L.psmooth, L.h_desc, psm);
+            build_pieces(L.prestr, L.h_desc, pre);  // this level's cells, restricted into from level l - 1
+        }
         for (int p = 0; p < nprob; p++) {
             if (has[p]) L.all_cells += L.h_desc[p].n;
             if (smooth[p]) L.smooth_cells += L.h_desc[p].n;
@@ -1587,6 +1713,7 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
             L.idg32 = dalloc<float>(n, owned);
         } else {
             L.idg64 = dalloc<double>(n, owned);
+            L.dg64 = dalloc<double>(n, owned);
         }
         size_t vs = mixed ? sizeof(float) : sizeof(double);
         for (int k = 0; k < 4; k++) L.work[k] = dalloc<char>(n * vs, owned);
@@ -1658,7 +1785,15 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
     }
     // state, reductions, coarse factors
     d_state = dalloc<CgState>(nprob, owned);
-    d_count = dalloc<int>(4, owned);
+    // active problems, -, loop passes, -; behind them the persistent kernel's barrier words
+    d_count = dalloc<int>(kCountWords, owned);
+    if (persist_blocks) {
+        std::vector<int2> pt(nprob);
+        for (int p = 0; p < nprob; p++) pt[p] = make_int2(ptail[p], nlev[p] - 1);
+        d_ptail = dalloc<int2>(nprob, owned);
+        d_ppart = dalloc<double2>(2 * (size_t)std::max(pall.n, lv[0].psmooth.n), owned);
+        CK(cudaMemcpy(d_ptail, pt.data(), nprob * sizeof(int2), cudaMemcpyHostToDevice));
+    }
     d_factor_status = dalloc<int>(2, owned);
     CK(cudaMemset(d_factor_status, 0, 2 * sizeof(int)));
     rs.partials = dalloc<double2>(std::max(maxblocks, 1), owned);
@@ -1766,6 +1901,8 @@ StructBatch::~StructBatch() {
     cudaStreamSynchronize(stream);  // then `owned` and `pinned` free the buffers
 }
 
+constexpr int kCountBar = 32;  // the barrier words' place behind the counts
+static_assert(kCountWords >= kCountBar + kGridBarWords, "barrier words");
 static inline unsigned nb_of(const BlockMap &m) { return (unsigned)m.nblocks; }
 
 // ---- assembly and hierarchy
@@ -1773,11 +1910,11 @@ template <typename T>
 static Coeffs<T> coeffs_of(StructBatch::Level &L, bool mixed);
 template <>
 Coeffs<double> coeffs_of<double>(StructBatch::Level &L, bool) {
-    return Coeffs<double>{L.c64[0], L.c64[1], L.c64[2], L.c64[3], L.idg64};
+    return Coeffs<double>{L.c64[0], L.c64[1], L.c64[2], L.c64[3], L.idg64, L.dg64};
 }
 template <>
 Coeffs<float> coeffs_of<float>(StructBatch::Level &L, bool) {
-    return Coeffs<float>{L.c16[0], L.c16[1], L.c16[2], L.c16[3], L.idg32};
+    return Coeffs<float>{L.c16[0], L.c16[1], L.c16[2], L.c16[3], L.idg32, nullptr};
 }
 
 // The fused tail's per-level pointer table, written once at construction: staged in pinned
@@ -1853,7 +1990,7 @@ void StructBatch::assemble(const double *Ks, const double *kc, int kind, const d
             KTimer _kt(this, kname("k_invdiag", l, false), L.all_cells);
             k_invdiag<<<nb_of(L.all), kBlock, 0, stream>>>(L.d_desc, L.all.d_map, coeffs_of<double>(L, false),
                                                            mixed ? coeffs_of<float>(L, true) : Coeffs<float>{},
-                                                           mixed ? nullptr : L.idg64, mixed ? L.idg32 : nullptr);
+                                                           mixed ? nullptr : L.idg64, mixed ? nullptr : L.dg64, mixed ? L.idg32 : nullptr);
         }
         LAUNCH_CHECK();
     }
@@ -2593,6 +2730,77 @@ void StructBatch::df_pcg(const double *b64, double *x64, double tol2) {
     }
 }
 
+// ---- the whole solve in one launch (dpf_persist.cuh)
+// Mixed handles with a finest level of 2^21 cells or more keep the plane kernels, which stage whole
+// planes and run near the copy rate; everything else is bound by its steps' latency (or, in FP64, by
+// the FP64 pipe, which the persistent kernel's passes use less). Per-kernel profiles, host-driven loops
+// and the cluster tail ask for the separate kernels.
+bool StructBatch::use_persist() const {
+    if (!persist_blocks || !opt.use_graphs || prof_on || opt.tail_cluster > 1) return false;
+    return !mixed || (!lv[0].pm.ok && N < (1LL << 21));
+}
+
+template <typename T>
+void StructBatch::solve_persistent(const double *b, double *x, double tol2) {
+    PersistParams<T> P{};
+    auto segs = [](const Pieces &q) { return PersistSegs{q.list, q.pinfo, q.n}; };
+    for (int l = 0; l < nlev_max; l++) {
+        Level &L = lv[l];
+        P.lv[l] = PersistLevel<T>{L.d_desc, coeffs_of<T>(L, mixed), (T *)L.work[0], (T *)L.work[1], (T *)L.work[2],
+                                  (T *)L.work[3], L.dir, segs(L.psmooth),
+                                  l + 1 < nlev_max ? segs(lv[l + 1].prestr) : PersistSegs{}};
+    }
+    P.nlev = nlev_max;
+    P.nprob = nprob;
+    P.invtheta = (T)inv_theta;
+    P.scale = (T)opt.coarse_scale;
+    P.deg = opt.cheb_degree;
+    for (int p = 0; p < nprob; p++) P.onelevel |= nlev[p] == 1;
+    for (int k = 0; k < P.deg; k++) {
+        P.c1[k] = (T)cheb_c1[k];
+        P.c2[k] = (T)cheb_c2[k];
+    }
+    P.u1 = P.deg > 1 ? (T(1) + P.c1[1]) * P.invtheta : T(0);
+    P.all = segs(pall);
+    P.tail = d_ptail;
+    P.Inv = d_coarseL;
+    P.st = d_state;
+    P.count = d_count;
+    P.bar = (unsigned *)d_count + kCountBar;
+    P.expired = d_factor_status + 1;
+    P.partials = d_ppart;
+    P.nslots = std::max(pall.n, lv[0].psmooth.n);
+    P.tol2 = tol2;
+    P.maxiter = opt.maxiter;
+    P.max_rounds = opt.max_outer;
+    P.zero_guess = zero_guess ? 1 : 0;
+    P.b64 = b;
+    P.x64 = x;
+    P.r = (T *)cgv[0];
+    P.z = (T *)cgv[1];
+    P.p = mixed ? nullptr : (double *)cgv[2];
+    P.q = mixed ? nullptr : (double *)cgv[3];
+    P.r64 = r64;
+    P.rd = dfv[1];
+    P.pd = dfv[2];
+    P.qd = dfv[3];
+    P.cdf = CoeffsDF{cdf[0], cdf[1], cdf[2], cdf[3]};
+    P.C64 = coeffs_of<double>(lv[0], true);
+    CK(cudaMemsetAsync(d_count, 0, kCountWords * sizeof(int), stream));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(persist_blocks);
+    cfg.blockDim = dim3(kPersistThreads);
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    KTimer _kt(this, kname("k_solve_persistent", 0, sizeof(T) == 4), lv[0].all_cells);
+    CK(nprob == 1 ? cudaLaunchKernelEx(&cfg, k_solve_persistent<T, true>, P)
+                  : cudaLaunchKernelEx(&cfg, k_solve_persistent<T, false>, P));
+}
+
 // ---- full solve of A x = b for every problem (x holds the initial guess)
 void StructBatch::solve(const double *b, double *x, double reltol) {
     if (opt.solver == DPF_SOLVER_CHOLESKY && direct_solve(b, x)) return;
@@ -2602,7 +2810,8 @@ void StructBatch::solve(const double *b, double *x, double reltol) {
         bool &f;
         ~ZeroGuessReset() { f = false; }
     } zg{zero_guess};
-    {
+    const bool persist = use_persist();
+    if (!persist) {
         KTimer _kt(this, kname("k_state_init", 0, false), 0);
         launch_pdl(k_state_init, (nprob + 127) / 128, 128, 0, stream, d_state, nprob);
     }
@@ -2610,7 +2819,11 @@ void StructBatch::solve(const double *b, double *x, double reltol) {
     CK(cudaMemsetAsync(d_factor_status + 1, 0, sizeof(int), stream));  // expired-wait word of this solve
     graph_body_kernels = 0;
     stats_fresh = false;
-    if (!mixed) {
+    if (persist) {
+        if (mixed) solve_persistent<float>(b, x, tol2);
+        else solve_persistent<double>(b, x, tol2);
+        stats_outer = 0;
+    } else if (!mixed) {
         pcg<double>(b, x, tol2);
         stats_outer = 0;
     } else {
@@ -2640,7 +2853,7 @@ void StructBatch::solve(const double *b, double *x, double reltol) {
     }
     if (h_misc[1]) {
         last_status = DPF_TIMEOUT;
-        last_message = "a shared-memory staging wait of a smoother kernel expired";
+        last_message = "a bounded wait of a solver kernel (staging or grid barrier) expired";
     }
 }
 

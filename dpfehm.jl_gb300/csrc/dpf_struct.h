@@ -70,7 +70,15 @@ public:
         int halo = 0, cy = 0, slab = 0, coarse = 0;
         int halo2 = 0, cy2 = 0, coarse2 = 0;  // regions of the fused kernels (two halo rows)
     };
+    // pieces of the persistent solve kernel (dpf_persist.cuh): per problem that takes part, equal shares
+    // of its cells; list entries {problem, piece, pieces, 0}, pinfo per problem {first, count}
+    struct Pieces {
+        int4 *list = nullptr;
+        int2 *pinfo = nullptr;
+        int n = 0;
+    };
     struct Level {
+        Pieces psmooth, prestr;  // cells of the smoothed problems; of their next level
         long long ntot = 0;
         long long all_cells = 0, smooth_cells = 0, coarse_cells = 0;
         std::vector<LevelDesc> h_desc;
@@ -87,7 +95,7 @@ public:
         long long csolve_cells = 0;
         uint8_t *dir = nullptr;        // identity (Dirichlet) rows
         double *c64[4] = {nullptr, nullptr, nullptr, nullptr};  // cx, cy, cz, leak
-        double *idg64 = nullptr;       // inverse diagonal (FP64 solves)
+        double *idg64 = nullptr, *dg64 = nullptr;  // inverse diagonal and diagonal (FP64 solves)
         __nv_bfloat16 *c16[4] = {nullptr, nullptr, nullptr, nullptr};  // FP32 V-cycle (bf16)
         float *idg32 = nullptr;        // inverse diagonal (FP32 V-cycle)
         void *work[4] = {nullptr, nullptr, nullptr, nullptr};   // xa, xb, b, d (V-cycle precision)
@@ -147,6 +155,15 @@ public:
     void choose_direct();
     std::unique_ptr<FrontSolver> fronts;
     bool direct_tried = false, direct_stale = true, direct_ok = false;
+    // one cooperative launch for the whole solve; use_persist: where it is the faster form
+    bool use_persist() const;
+    template <typename T>
+    void solve_persistent(const double *b, double *x, double tol2);
+    void build_pieces(Pieces &P, const std::vector<LevelDesc> &desc, const std::vector<int> &take);
+    Pieces pall;                     // finest cells of every problem
+    int2 *d_ptail = nullptr;         // per problem {first level of its one-block tail, coarsest level}
+    double2 *d_ppart = nullptr;      // its reduction slots
+    int persist_blocks = 0;          // blocks of the cooperative launch (0: not available)
     cudaGraphExec_t loop_graph(int kind, void *x);
     void run_loop(int kind, void *x);
     int read_count(int which);

@@ -238,7 +238,9 @@ __device__ __forceinline__ void apply7(const LevelDesc &L, const Cell &c, const 
     const long long i = c.i;
     const long long sy = L.nz, sx = (long long)L.ny * L.nz;
     T lk = cf(C.leak[i]);
-    T a = lk * xi, d = lk;
+    T a, d = lk;
+    if constexpr (sizeof(T) == 8) a = __double_as_longlong(lk) << 1 ? lk * xi : T(0);  // 0 beside no Dirichlet cell
+    else a = lk * xi;
 #if DPF_CHECKED
     // every neighbour the flags below admit lies inside the problem's cells
     if (!(DPF_INSIDE(CK_NEIGHBOUR, c.iz + 1 < L.nz ? i + 1 : i, L.off, L.off + L.n) &&
@@ -260,6 +262,42 @@ __device__ __forceinline__ void apply7(const LevelDesc &L, const Cell &c, const 
     if (c.ix > 0)        { T w = cf(C.cx[i - sx]); a += w * (xi - xat(i - sx, c.ix - 1, c.iy, c.iz));  d += w; }
     Ax = a;
     diag = d;
+}
+
+// b_i - (A x)_i for the V-cycle. FP32 levels: from apply7 (the diagonal comes with it, for the
+// smoother's division). FP64 levels: b - dg x_i + sum_f c_f x_j with the stored diagonal, 7 FP64
+// instructions against 14: GB300 issues 1.6 of them per clock and SM, which bounds every FP64 smoother. The
+// cancellation that the flux form avoids is in the last bits of diag_i x_i, and the V-cycle only
+// preconditions: CG's own products and residuals keep the flux form.
+template <typename T, typename XAt>
+__device__ __forceinline__ T resid7(const LevelDesc &L, const Cell &c, const Coeffs<T> &C, T bi, T xi, XAt xat,
+                                    T &diag) {
+    if constexpr (sizeof(T) == 8) {
+        const long long i = c.i;
+        const long long sy = L.nz, sx = (long long)L.ny * L.nz;
+        diag = T(0);
+        T r = fma(-C.dg[i], xi, bi);
+#if DPF_CHECKED
+        if (!(DPF_INSIDE(CK_NEIGHBOUR, c.iz + 1 < L.nz ? i + 1 : i, L.off, L.off + L.n) &&
+              DPF_INSIDE(CK_NEIGHBOUR, c.iz > 0 ? i - 1 : i, L.off, L.off + L.n) &&
+              DPF_INSIDE(CK_NEIGHBOUR, c.iy + 1 < L.ny ? i + sy : i, L.off, L.off + L.n) &&
+              DPF_INSIDE(CK_NEIGHBOUR, c.iy > 0 ? i - sy : i, L.off, L.off + L.n) &&
+              DPF_INSIDE(CK_NEIGHBOUR, c.ix + 1 < L.nx ? i + sx : i, L.off, L.off + L.n) &&
+              DPF_INSIDE(CK_NEIGHBOUR, c.ix > 0 ? i - sx : i, L.off, L.off + L.n)))
+            return r;
+#endif
+        if (c.iz + 1 < L.nz) r = fma(C.cz[i], xat(i + 1, c.ix, c.iy, c.iz + 1), r);
+        if (c.iz > 0) r = fma(C.cz[i - 1], xat(i - 1, c.ix, c.iy, c.iz - 1), r);
+        if (c.iy + 1 < L.ny) r = fma(C.cy[i], xat(i + sy, c.ix, c.iy + 1, c.iz), r);
+        if (c.iy > 0) r = fma(C.cy[i - sy], xat(i - sy, c.ix, c.iy - 1, c.iz), r);
+        if (c.ix + 1 < L.nx) r = fma(C.cx[i], xat(i + sx, c.ix + 1, c.iy, c.iz), r);
+        if (c.ix > 0) r = fma(C.cx[i - sx], xat(i - sx, c.ix - 1, c.iy, c.iz), r);
+        return r;
+    } else {
+        T Ax;
+        apply7(L, c, C, xi, xat, Ax, diag);
+        return bi - Ax;
+    }
 }
 
 // |v| as a float, truncated, from v's bits (integer operations only): 0 below 2^-126, 3e38 at or

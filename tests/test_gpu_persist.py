@@ -1,0 +1,59 @@
+"""The one-launch solve (the persistent kernel) against the oracle and against the separate kernels
+(use_graphs = 0), at the sizes where its parts meet: grids of a single level (up to 64 cells), levels on
+both sides of the one-block tail's limits (512 cells in FP64, 2048 in FP32), one-cell-thick and odd axes,
+every parity of the smoothing degree, and batches with fewer and with more problems than shares.
+Tolerances: heads 1e-8 and gradients 1e-6 of the oracle's, and 1e-10 / 1e-8 between the two paths (their
+V-cycles agree to rounding, and both solve to 1e-12)."""
+import numpy as np
+import pytest
+
+from helpers import rel, steady_case
+
+pytestmark = pytest.mark.gpu
+
+
+def _solve(pkg, cases, **opt):
+    B = pkg.GroundwaterBatch([c["ns"] for c in cases], [c["mins"] for c in cases], [c["maxs"] for c in cases],
+                             [c["dn"] for c in cases], reltol=1e-12, **opt)
+    cat = lambda k: np.concatenate([c[k] for c in cases])
+    obs = [np.arange(0, c["N"], 3) for c in cases]
+    h, g = B.solve_grad_logk(cat("logK"), cat("dh"), cat("Qs"), obs)
+    return B, obs, np.asarray(h), np.asarray(g)
+
+
+def _check(pkg, orc, cases, **opt):
+    B, obs, h, g = _solve(pkg, cases, **opt)
+    B0, _, h0, g0 = _solve(pkg, cases, use_graphs=0, **opt)
+    assert B.launch_count < B0.launch_count  # one launch per solve
+    off = B.cell_offsets
+    for k, c in enumerate(cases):
+        s = slice(off[k], off[k + 1])
+        O = orc.Problem(c["N"], c["nb"], c["aol"], c["dn"])
+        ho = O.steady(orc.logk_to_faces(c["nb"], c["logK"]), c["dh"], c["Qs"], reltol=1e-14)
+        d = np.zeros(c["N"])
+        np.add.at(d, obs[k], 2 * ho[obs[k]])
+        go = orc.logk_to_faces_vjp(c["nb"], c["logK"], O.adjoint(c["dh"], d, reltol=1e-14)[0])
+        assert rel(h[s], ho) < 1e-8 and rel(g[s], go) < 1e-6, k
+        assert rel(h[s], h0[s]) < 1e-10 and rel(g[s], g0[s]) < 1e-8, k
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("ns", [(4, 4, 4), (5, 13, 1), (1, 1, 70), (16, 16, 16), (17, 16, 16), (33, 9, 7),
+                                (26, 25, 26), (51, 2, 43)])
+def test_one_grid(gpu_lib, orc, ns, precision):
+    _check(gpu_lib, orc, [steady_case(gpu_lib, ns, ell=4.0, sigma=1.0, seed=sum(ns), ndir=2, nq=2)], precision=precision)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("degree", [1, 3, 4])
+def test_smoothing_degrees(gpu_lib, orc, degree, precision):
+    _check(gpu_lib, orc, [steady_case(gpu_lib, (21, 18, 9), sigma=1.0, seed=3, ndir=1, nq=2)], precision=precision,
+           cheb_degree=degree)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("shapes", [[(4, 4, 3), (20, 17, 9), (40, 6, 5)], [(3, 3, 3), (5, 4, 3)],
+                                    [(6, 5, 4)] * 90 + [(24, 20, 10)]])
+def test_batches(gpu_lib, orc, shapes, precision):
+    cases = [steady_case(gpu_lib, ns, sigma=1.0, seed=k % 7, ndir=1 + k % 2, nq=2) for k, ns in enumerate(shapes)]
+    _check(gpu_lib, orc, cases, precision=precision)
