@@ -144,11 +144,13 @@ __global__ void kg_coarse_leak(int nc, const int *__restrict__ mrp, const int *_
 }
 
 __global__ void kg_invdiag(int n, const int *__restrict__ rp, const double *__restrict__ v,
-                           const double *__restrict__ leak, double *__restrict__ idg64, float *__restrict__ idg32) {
+                           const double *__restrict__ leak, double *__restrict__ idg64, double *__restrict__ dg64,
+                           float *__restrict__ idg32) {
     GSTRIDE(i, n) {
         double d = leak[i];
         for (int e = rp[i]; e < rp[i + 1]; e++) d += v[e];
         double g = 1.0 / d;
+        if (dg64) dg64[i] = d;
         if (idg64) idg64[i] = g;
         if (idg32) idg32[i] = (float)g;
     }
@@ -663,6 +665,10 @@ __global__ void kg_dh0(int n, const uint8_t *__restrict__ dir, const double *__r
     GSTRIDE(i, n) out[i] = dir[i] ? 0.0 : shift[i] * mu[i];
 }
 
+}  // namespace dpf
+#include "dpf_gpersist.cuh"
+namespace dpf {
+
 // ================================================================ host side
 static void gck(cudaError_t e, const char *what) {
     if (e != cudaSuccess) {
@@ -844,6 +850,18 @@ GeneralSolver::GeneralSolver(long long N_, long long F_, const int64_t *a, const
     rs.tickets = dev<unsigned>(1);
     rs.capacity = nblocks;
     GCK(cudaMemsetAsync(rs.tickets, 0, sizeof(unsigned), stream));
+    {
+        // the persistent solve: one block per SM, all resident
+        int coop = 0, occ = 0;
+        GCK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev_id));
+        GCK(mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kg_solve_persistent<float>, kGpThreads, 0)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kg_solve_persistent<double>, kGpThreads, 0));
+        if (coop && occ >= 1 && (int)lv.size() <= kGpLevels) {
+            persist_blocks = sms;
+            d_bar = dev<unsigned>(kGridBarWords + 1);  // the barrier's words, then the expired-wait word
+            d_slots = dev<double2>(2 * (size_t)sms);
+        }
+    }
     dense_inv = dev<double>(kMaxCoarse * kMaxCoarse);
     h_count = (int *)pinned.alloc(4 * sizeof(int));
     h_state = (CgState *)pinned.alloc(sizeof(CgState));
@@ -1066,8 +1084,9 @@ void GeneralSolver::build_hierarchy() {
             L.idg32 = dev<float>(L.n);
         } else {
             L.idg64 = dev<double>(L.n);
+            L.dg64 = dev<double>(L.n);
         }
-        for (int k = 0; k < 4; k++) L.work[k] = dev<char>(L.n * vs);
+        for (int k = 0; k < 5; k++) L.work[k] = dev<char>(L.n * vs);
     }
 }
 
@@ -1105,7 +1124,7 @@ void GeneralSolver::assemble(const double *Ks, const double *kc, int kind, const
         GLAUNCH();
     }
     for (auto &L : lv) {
-        kg_invdiag<<<gblocks(L.n, nblocks), kBlock, 0, stream>>>(L.n, L.rp, L.v64, L.leak64, L.idg64, L.idg32);
+        kg_invdiag<<<gblocks(L.n, nblocks), kBlock, 0, stream>>>(L.n, L.rp, L.v64, L.leak64, L.idg64, L.dg64, L.idg32);
         GLAUNCH();
         if (mixed) {
             kg_to_float<<<gblocks(L.nnz, nblocks), kBlock, 0, stream>>>(L.nnz, L.v64, L.v32);
@@ -1359,16 +1378,89 @@ bool GeneralSolver::direct_solve(const double *b, double *x) {
     return true;
 }
 
+// ---- the whole solve in one launch (dpf_gpersist.cuh)
+template <typename T>
+void GeneralSolver::solve_persistent(const double *b, double *x, double tol2) {
+    GpParams<T> P{};
+    P.nl = (int)lv.size();
+    P.tail = P.nl;
+    for (int l = 0; l < P.nl; l++) {
+        GLevel &L = lv[l];
+        const GOp<T> A = gop<T>(L);
+        P.lv[l] = GpLevel<T>{L.n, L.rp, L.ci, L.agg, L.mrp, L.mci, A.v, A.leak, A.idg,
+                             sizeof(T) == 8 ? (const T *)L.dg64 : nullptr, (T *)L.work[0], (T *)L.work[1],
+                             (T *)L.work[2], (T *)L.work[3], (T *)L.work[4], L.dir};
+        if (l >= 1 && L.n <= kGpTail && P.tail == P.nl) P.tail = l;
+    }
+    P.deg = opt.cheb_degree;
+    P.dense = lv.back().dense ? 1 : 0;
+    for (int k = 0; k < P.deg; k++) {
+        P.c1[k] = (T)cheb_c1[k];
+        P.c2[k] = (T)cheb_c2[k];
+    }
+    for (int k = 0; k < 8; k++) {
+        P.e1[k] = (T)cheb8_c1[k];
+        P.e2[k] = (T)cheb8_c2[k];
+    }
+    P.invtheta = (T)inv_theta;
+    P.scale = (T)opt.coarse_scale;
+    P.Inv = dense_inv;
+    P.st = d_state;
+    P.bar = d_bar;
+    P.expired = (int *)d_bar + kGridBarWords;
+    P.partials = d_slots;
+    P.tol2 = tol2;
+    P.maxiter = opt.maxiter;
+    P.max_rounds = opt.max_outer;
+    P.dir = lv[0].dir;
+    P.b64 = b;
+    P.x64 = x;
+    P.r = (T *)cgv[0];
+    P.z = (T *)cgv[1];
+    P.p = mixed ? nullptr : (double *)cgv[2];
+    P.q = mixed ? nullptr : (double *)cgv[3];
+    P.r64 = r64;
+    P.rd = dfv[1];
+    P.pd = dfv[2];
+    P.qd = dfv[3];
+    P.vdf = vdf;
+    P.leakdf = leakdf;
+    P.v64 = lv[0].v64;
+    P.leak64 = lv[0].leak64;
+    GCK(cudaMemsetAsync(d_bar, 0, (kGridBarWords + 1) * sizeof(unsigned), stream));
+    cudaLaunchAttribute at[1];
+    at[0].id = cudaLaunchAttributeCooperative;
+    at[0].val.cooperative = 1;
+    cudaLaunchConfig_t cfg = {};
+    cfg.gridDim = dim3(persist_blocks);
+    cfg.blockDim = dim3(kGpThreads);
+    cfg.stream = stream;
+    cfg.attrs = at;
+    cfg.numAttrs = 1;
+    GCK(cudaLaunchKernelEx(&cfg, kg_solve_persistent<T>, P));
+    launches++;
+    from_dev(h_count + 2, d_bar + kGridBarWords, sizeof(int));
+}
+
 void GeneralSolver::solve(const double *b, double *x) {
     if (opt.solver == DPF_SOLVER_CHOLESKY && direct_solve(b, x)) return;
     NvtxRange range("CG + AMG solve (CSR)");
-    kg_state_init<<<1, 1, 0, stream>>>(d_state);
-    GLAUNCH();
     const double tol2 = opt.reltol * opt.reltol;
-    if (!mixed) pcg<double>(b, x, tol2);
-    else df_pcg(b, x, tol2);
+    // one launch, except where per-kernel profiles or host-driven loops are asked for
+    const bool persist = persist_blocks && opt.use_graphs && !prof_on;
+    h_count[2] = 0;
+    if (persist) {
+        if (mixed) solve_persistent<float>(b, x, tol2);
+        else solve_persistent<double>(b, x, tol2);
+    } else {
+        kg_state_init<<<1, 1, 0, stream>>>(d_state);
+        GLAUNCH();
+        if (!mixed) pcg<double>(b, x, tol2);
+        else df_pcg(b, x, tol2);
+    }
     from_dev(h_state, d_state, sizeof(CgState));
     GCK(cudaStreamSynchronize(stream));
+    if (h_count[2]) h_state->status = DPF_TIMEOUT;
     stats_iters = h_state->total_iters;
     stats_outer = mixed ? h_state->outer : 0;
     stats_relres = mixed ? (h_state->obb > 0 ? std::sqrt(h_state->orr / h_state->obb) : 0.0)
@@ -1385,7 +1477,9 @@ int GeneralSolver::finish_status() {
         return DPF_BAD_INPUT;
     }
     if (h_state->status != DPF_OK)
-        last_message = h_state->status == DPF_NOT_CONVERGED ? "CG did not converge within maxiter" : "non-finite residual";
+        last_message = h_state->status == DPF_NOT_CONVERGED ? "CG did not converge within maxiter"
+                       : h_state->status == DPF_TIMEOUT     ? "a bounded wait of the solver kernel expired"
+                                                            : "non-finite residual";
     return h_state->status;
 }
 

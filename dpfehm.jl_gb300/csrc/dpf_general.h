@@ -18,14 +18,14 @@ namespace dpf {
 struct GLevel {
     int n = 0, nnz = 0;
     int *rp = nullptr, *ci = nullptr;        // couplings (no diagonal)
-    double *v64 = nullptr, *leak64 = nullptr, *idg64 = nullptr;
+    double *v64 = nullptr, *leak64 = nullptr, *idg64 = nullptr, *dg64 = nullptr;
     float *v32 = nullptr, *leak32 = nullptr, *idg32 = nullptr;
     uint8_t *dir = nullptr;                   // identity rows
     // transfer to the next coarser level
     int *agg = nullptr;                       // fine cell -> aggregate (-1: none)
     int *mrp = nullptr, *mci = nullptr;       // aggregate -> member cells (next level's row order)
     int *crp = nullptr, *cci = nullptr;       // coarse coupling -> contributing fine couplings
-    void *work[4] = {nullptr, nullptr, nullptr, nullptr};  // xa, xb, b, d
+    void *work[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};  // xa, xb, b, d, u = b D^-1
     bool dense = false;                       // coarsest level solved by its dense inverse
 };
 
@@ -97,6 +97,11 @@ private:
     template <typename T>
     void pcg(const T *b, T *x, double tol2);
     void df_pcg(const double *b64, double *x64, double tol2);
+    template <typename T>
+    void solve_persistent(const double *b, double *x, double tol2);  // the whole solve as one launch
+    int persist_blocks = 0;        // its blocks (0: not available)
+    unsigned *d_bar = nullptr;
+    double2 *d_slots = nullptr;
     void adjoint_solve(const double *delta_dev);
     int finish_status();
     int read_active();

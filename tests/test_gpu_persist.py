@@ -57,3 +57,38 @@ def test_smoothing_degrees(gpu_lib, orc, degree, precision):
 def test_batches(gpu_lib, orc, shapes, precision):
     cases = [steady_case(gpu_lib, ns, sigma=1.0, seed=k % 7, ndir=1 + k % 2, nq=2) for k, ns in enumerate(shapes)]
     _check(gpu_lib, orc, cases, precision=precision)
+
+
+def _mesh(kind):
+    """(cells, faces, Dirichlet cells): a shuffled grid, a random tree, or pairs of cells beside a Dirichlet one
+    (nothing to coarsen)."""
+    rng = np.random.default_rng(len(kind))
+    if kind.startswith("grid"):
+        nx, ny = (7, 6) if kind == "grid42" else (23, 23) if kind == "grid529" else (70, 51)
+        i = np.arange(nx * ny).reshape(nx, ny)
+        nb = np.concatenate([np.stack([i[:-1].ravel(), i[1:].ravel()], 1), np.stack([i[:, :-1].ravel(), i[:, 1:].ravel()], 1)])
+        return nx * ny, nb[rng.permutation(len(nb))], np.array([0, nx * ny - 1])
+    if kind == "tree":
+        k = np.arange(1, 900)
+        return 900, np.stack([(rng.random(899) * k).astype(np.int64), k], 1), np.array([0, 17])
+    k = np.arange(200)
+    return 300, np.stack([k, 200 + k // 2], 1), np.arange(200, 300)
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("kind,degree", [("grid42", 0), ("grid529", 0), ("grid529", 1), ("grid3570", 2), ("grid3570", 4),
+                                         ("tree", 0), ("pairs", 0)])
+def test_face_lists(gpu_lib, orc, kind, degree, precision):
+    n, nb, dn = _mesh(kind)
+    rng = np.random.default_rng(5)
+    aol, Ks = rng.uniform(0.5, 2.0, len(nb)), np.exp(-9.0 + rng.standard_normal(len(nb)))
+    dh, Qs, delta = np.zeros(n), np.zeros(n), rng.standard_normal(n)
+    dh[dn] = rng.uniform(0, 1, len(dn))
+    Qs[rng.choice(np.setdiff1d(np.arange(n), dn), 3, replace=False)] = [1e-4, 5e-5, -2e-5]
+    P = gpu_lib.GroundwaterProblem(nb, aol, dn, N=n, general=True, precision=precision, reltol=1e-12, cheb_degree=degree)
+    O = orc.Problem(n, nb, aol, dn)
+    want = (O.steady(Ks, dh, Qs, reltol=1e-14),) + tuple(O.adjoint(dh, delta, reltol=1e-14))
+    got = (P.forward(Ks, dh, Qs),) + tuple(P.adjoint(delta))
+    assert rel(got[0], want[0]) < 1e-8
+    for g, w in zip(got[1:], want[1:]):
+        assert rel(g, w) < 1e-6
