@@ -1104,14 +1104,17 @@ bool GeneralSolver::check_due(int it) const {
 
 static unsigned gblocks(long long n, int cap) { return (unsigned)std::max(1LL, std::min((n + kBlock - 1) / kBlock, (long long)cap)); }
 
-void GeneralSolver::assemble(const double *Ks, const double *kc, int kind, const double *shift_, bool init_x) {
+void GeneralSolver::assemble(const double *Ks, const double *kc, int kind, const double *shift_, bool init_x, bool same_op) {
     GLevel &L0 = lv[0];
-    direct_stale = true;  // a direct factor of the previous operator is out of date
-    choose_direct();
+    if (!same_op) {
+        direct_stale = true;  // a direct factor of the previous operator is out of date
+        choose_direct();
+    }
     const int n = (int)N;
     kg_assemble<<<gblocks(n, nblocks), kBlock, 0, stream>>>(n, irp, ifc, fa, fb, faol, Ks, kc, kind, L0.dir, in_dh, in_Q,
                                                            shift_, L0.leak64, b64, h, init_x ? 1 : 0);
     GLAUNCH();
+    if (same_op) return;
     kg_entry_vals<<<gblocks(L0.nnz, nblocks), kBlock, 0, stream>>>(L0.nnz, e_face, fa, fb, faol, Ks, kc, kind, L0.v64);
     GLAUNCH();
     GCK(cudaMemsetAsync(d_status, 0, sizeof(int), stream));

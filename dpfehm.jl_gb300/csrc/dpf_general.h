@@ -84,7 +84,7 @@ private:
     void setup_topology(const int64_t *a, const int64_t *b, const double *aol, const double *volumes, long long nd,
                         const int64_t *dn);
     void build_hierarchy();
-    void assemble(const double *Ks, const double *kc, int kind, const double *shift, bool init_x);
+    void assemble(const double *Ks, const double *kc, int kind, const double *shift, bool init_x, bool same_op = false);
     void solve(const double *b, double *x);
     // options.solver = DPF_SOLVER_CHOLESKY: x = A^-1 b by a factor of the FP64 operator (factored again
     // after each assembly); false when the system is too large for it (the iterative solve then runs)
@@ -120,7 +120,7 @@ private:
     void richards_buffers();
     void richards_stage(const double *Ks, const double *dpsi, const double *z, const double *alphas,
                         const double *Ns, const double *Qs, const double *psi0);
-    int richards_spd_solve(const double *rhs_dev, double *x_dev, const double *shift_dev);
+    int richards_spd_solve(const double *rhs_dev, double *x_dev, const double *shift_dev, bool same_op = false);
     int richards_nonlinear(const double *shift_dev, const double *psi_old, double tol, int maxit, int &iters,
                            double &relres);
     int richards_gmres(const double *rhs_dev, double *x_dev, const double *shift_dev, double tol, int maxit,

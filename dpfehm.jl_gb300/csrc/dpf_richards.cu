@@ -34,42 +34,55 @@ constexpr int kRBlock = 256;
 
 #define RSTRIDE(i, n) for (int i = blockIdx.x * blockDim.x + threadIdx.x; i < (n); i += gridDim.x * blockDim.x)
 
-// van Genuchten kr(psi; alpha, N) and its derivatives by psi, alpha and N (psi >= 0: kr = 1)
+// van Genuchten kr(psi; alpha, N) and, as far as kWant asks, its derivatives (psi >= 0: kr = 1)
+enum KrWant { kKrValue, kKrPsi, kKrAll };
 struct Kr {
     double v, dpsi, dalpha, dN;
 };
 
+// FP64 arithmetic bounds the kernels that evaluate it (pow is ~100 FP64 instructions, and a B300 SM issues
+// 1.6 a clock): two powers per value, with u^N = u u^(N-1) and A^(-m/2) = sqrt(A^-m), and derivatives only
+// where they are used. With a power for each, and the derivatives always formed, the faces of a 200k-cell
+// grid (597k faces, two values each) took 895 us. u^(N-1) is the rounded one: N - 1 is exact for N >= 1/2,
+// and where u^N underflows u^(N-1) / u is still the right limit.
+template <KrWant kWant>
 __device__ Kr kr_vg(double psi, double alpha, double N) {
     Kr k{1.0, 0.0, 0.0, 0.0};
     if (!(psi < 0.0)) return k;
     const double m = (N - 1.0) / N;
     const double ap = fabs(alpha * psi);                 // u
-    const double uN = pow(ap, N), uN1 = pow(ap, N - 1.0);
+    const double uN1 = pow(ap, N - 1.0);
+    const double uN = ap > 0.0 ? uN1 * ap : pow(ap, N);
     const double A = 1.0 + uN;
     const double Am = pow(A, -m);
     const double numer = 1.0 - uN1 * Am;
-    const double Amh = pow(A, -0.5 * m);
+    const double Amh = sqrt(Am);
     k.v = numer * numer * Amh;
+    if (kWant == kKrValue) return k;
     // by u: d numer = -(N-1) u^(N-2) A^-m + m N u^(2N-2) A^(-m-1); d A = N u^(N-1)
+    const double rA = 1.0 / A;
     const double uN2 = ap > 0.0 ? uN1 / ap : 0.0;
-    const double dnum_du = -(N - 1.0) * uN2 * Am + m * N * uN1 * uN1 * Am / A;
-    const double dkr_du = 2.0 * numer * dnum_du * Amh - 0.5 * m * numer * numer * Amh / A * N * uN1;
+    const double dnum_du = -(N - 1.0) * uN2 * Am + m * N * uN1 * uN1 * Am * rA;
+    const double dkr_du = 2.0 * numer * dnum_du * Amh - 0.5 * m * numer * numer * Amh * rA * N * uN1;
     k.dpsi = dkr_du * (-alpha);   // u = -alpha psi for psi < 0, alpha > 0
+    if (kWant == kKrPsi) return k;
     k.dalpha = dkr_du * fabs(psi);
     // by N (m = 1 - 1/N, dm/dN = 1/N^2); u^N and u^(N-1) gain a factor ln u
     if (ap > 0.0) {
         const double lu = log(ap), lA = log(A), dm = 1.0 / (N * N);
         const double dA = uN * lu;
-        const double dAm = Am * (-dm * lA - m * dA / A);
+        const double dAm = Am * (-dm * lA - m * dA * rA);
         const double dnum = -(uN1 * lu * Am + uN1 * dAm);
-        const double dAmh = Amh * (-0.5 * dm * lA - 0.5 * m * dA / A);
+        const double dAmh = Amh * (-0.5 * dm * lA - 0.5 * m * dA * rA);
         k.dN = 2.0 * numer * dnum * Amh + numer * numer * dAmh;
     }
     return k;
 }
 
-// Per face: Picard conductance K hm (kr_a, kr_b), the flux-derivative parts of the Jacobian
-// (na, nb) and the face difference of the total head.
+// Per face: Picard conductance K hm (kr_a, kr_b) and, with kJac, the flux-derivative parts of the Jacobian
+// (na, nb) and the face difference of the total head. FP64 arithmetic bounds it (see kr_vg): 597k faces
+// 448 us without the Jacobian and 527 us with it (895 us with the six powers and all derivatives).
+template <bool kJac>
 __global__ void kr_faces(int F, const int *__restrict__ fa, const int *__restrict__ fb,
                          const double *__restrict__ aol, const double *__restrict__ Ks,
                          const double *__restrict__ alphas, const double *__restrict__ Ns,
@@ -77,15 +90,16 @@ __global__ void kr_faces(int F, const int *__restrict__ fa, const int *__restric
                          double *__restrict__ na, double *__restrict__ nb) {
     RSTRIDE(f, F) {
         const int a = fa[f], b = fb[f];
-        const Kr ka = kr_vg(psi[a], alphas[f], Ns[f]), kb = kr_vg(psi[b], alphas[f], Ns[f]);
+        constexpr KrWant want = kJac ? kKrPsi : kKrValue;
+        const Kr ka = kr_vg<want>(psi[a], alphas[f], Ns[f]), kb = kr_vg<want>(psi[b], alphas[f], Ns[f]);
         const double s = ka.v + kb.v;
         const double is = s > 0.0 ? 1.0 / s : 0.0;  // both kr zero: no conductance
         const double H = 2.0 * ka.v * kb.v * is;
-        const double dHa = 2.0 * kb.v * kb.v * is * is * ka.dpsi, dHb = 2.0 * ka.v * ka.v * is * is * kb.dpsi;
-        const double D = psi[b] + z[b] - psi[a] - z[a];
-        const double Ka = Ks[f] * aol[f];
         Kh[f] = Ks[f] * H;
-        if (na) {
+        if (kJac) {
+            const double dHa = 2.0 * kb.v * kb.v * is * is * ka.dpsi, dHb = 2.0 * ka.v * ka.v * is * is * kb.dpsi;
+            const double D = psi[b] + z[b] - psi[a] - z[a];
+            const double Ka = Ks[f] * aol[f];
             na[f] = Ka * dHa * D;
             nb[f] = -Ka * dHb * D;
         }
@@ -234,7 +248,7 @@ __global__ void richards_mu_step(int n, const double *__restrict__ mnew, double 
 }
 
 // Face gradients with mu = -lambda (0 at Dirichlet cells): dK_f = H aol D (mu_a - mu_b);
-// dalpha_f, dN_f = K aol D (mu_a - mu_b) dH/d(.)
+// dalpha_f, dN_f = K aol D (mu_a - mu_b) dH/d(.); bound by kr_vg's arithmetic (597k faces: 1000 -> 643 us)
 __global__ void richards_face_grads(int F, const int *__restrict__ fa, const int *__restrict__ fb,
                                     const double *__restrict__ aol, const double *__restrict__ Ks,
                                     const double *__restrict__ alphas, const double *__restrict__ Ns,
@@ -244,7 +258,7 @@ __global__ void richards_face_grads(int F, const int *__restrict__ fa, const int
                                     int accumulate) {
     RSTRIDE(f, F) {
         const int a = fa[f], b = fb[f];
-        const Kr ka = kr_vg(psi[a], alphas[f], Ns[f]), kb = kr_vg(psi[b], alphas[f], Ns[f]);
+        const Kr ka = kr_vg<kKrAll>(psi[a], alphas[f], Ns[f]), kb = kr_vg<kKrAll>(psi[b], alphas[f], Ns[f]);
         const double s = ka.v + kb.v;
         const double is = s > 0.0 ? 1.0 / s : 0.0;
         const double H = 2.0 * ka.v * kb.v * is;
@@ -259,12 +273,13 @@ __global__ void richards_face_grads(int F, const int *__restrict__ fa, const int
 }
 
 // dQ_j = mu_j at free cells; ddirichletpsis_k = delta_k + sum_{f=(j,k), j free} mu_j dF_jk/dpsi_k
-// at Dirichlet cells (dF_jk/dpsi_k = K aol (dH/dpsi_k D_jk + H))
+// at Dirichlet cells (dF_jk/dpsi_k = K aol (dH/dpsi_k D_jk + H)), from the conductances Kh and Jacobian parts
+// na, nb that kr_faces left at this psi. Memory-bound; evaluating kr again here put all of its arithmetic on
+// the few threads that hold a Dirichlet cell (380 us for 200k cells, 9 us now).
 __global__ void richards_cell_grads(int n, const int *__restrict__ irp, const int *__restrict__ ifc,
                                     const int *__restrict__ fa, const int *__restrict__ fb,
-                                    const double *__restrict__ aol, const double *__restrict__ Ks,
-                                    const double *__restrict__ alphas, const double *__restrict__ Ns,
-                                    const double *__restrict__ psi, const double *__restrict__ z,
+                                    const double *__restrict__ aol, const double *__restrict__ Kh,
+                                    const double *__restrict__ na, const double *__restrict__ nb,
                                     const uint8_t *__restrict__ dir, const double *__restrict__ mu,
                                     const double *__restrict__ delta, double *__restrict__ dQ,
                                     double *__restrict__ ddp, int accumulate) {
@@ -278,16 +293,11 @@ __global__ void richards_cell_grads(int n, const int *__restrict__ irp, const in
         double g = (accumulate ? ddp[k] : 0.0) + delta[k];
         for (int e = irp[k]; e < irp[k + 1]; e++) {
             const int f = ifc[e];
-            const int j = fa[f] == k ? fb[f] : fa[f];
+            const bool first = fa[f] == k;
+            const int j = first ? fb[f] : fa[f];
             if (!DPF_INSIDE(CK_NEIGHBOUR, j, 0, n)) continue;
             if (dir[j]) continue;
-            const Kr kk = kr_vg(psi[k], alphas[f], Ns[f]), kj = kr_vg(psi[j], alphas[f], Ns[f]);
-            const double s = kk.v + kj.v;
-            const double is = s > 0.0 ? 1.0 / s : 0.0;
-            const double H = 2.0 * kk.v * kj.v * is;
-            const double dHk = 2.0 * kj.v * kj.v * is * is * kk.dpsi;
-            const double Djk = psi[k] + z[k] - psi[j] - z[j];
-            g += mu[j] * Ks[f] * aol[f] * (dHk * Djk + H);
+            g += mu[j] * (Kh[f] * aol[f] - (first ? na[f] : nb[f]));
         }
         ddp[k] = g;
     }
@@ -411,11 +421,12 @@ void GeneralSolver::richards_buffers() {
 }
 
 // One SPD solve (shift + A(Kh)) x = rhs (x = 0 at Dirichlet cells) with the handle's CG + AMG;
-// shift = S V / dt in a backward-Euler step, null when steady.
-int GeneralSolver::richards_spd_solve(const double *rhs_dev, double *x_dev, const double *shift_dev) {
+// shift = S V / dt in a backward-Euler step, null when steady. same_op: the handle holds this operator
+// already (its hierarchy, or its factor, is kept; only the right-hand side is formed).
+int GeneralSolver::richards_spd_solve(const double *rhs_dev, double *x_dev, const double *shift_dev, bool same_op) {
     rck(cudaMemcpyAsync(in_Q, rhs_dev, N * sizeof(double), cudaMemcpyDeviceToDevice, stream), "rhs");
     rck(cudaMemcpyAsync(in_dh, rc_zero, N * sizeof(double), cudaMemcpyDeviceToDevice, stream), "dh");
-    assemble(rc_Kh, nullptr, 0, shift_dev, true);
+    assemble(rc_Kh, nullptr, 0, shift_dev, true, same_op);
     solve(b64, h);
     rck(cudaMemcpyAsync(x_dev, h, N * sizeof(double), cudaMemcpyDeviceToDevice, stream), "solution");
     rck(cudaStreamSynchronize(stream), "sync");
@@ -435,8 +446,8 @@ int GeneralSolver::richards_nonlinear(const double *shift_dev, const double *psi
     const unsigned nbF = rblocks(F, nblocks), nbN = rblocks(N, nblocks);
     double floor2 = 0.0;  // squared rounding floor of the last residual evaluated
     auto residual = [&]() -> double2 {
-        kr_faces<<<nbF, kRBlock, 0, stream>>>((int)F, fa, fb, faol, rc_Ks, rc_al, rc_N, rc_psi, rc_z, rc_Kh,
-                                              nullptr, nullptr);
+        kr_faces<false><<<nbF, kRBlock, 0, stream>>>((int)F, fa, fb, faol, rc_Ks, rc_al, rc_N, rc_psi, rc_z, rc_Kh,
+                                                     nullptr, nullptr);
         GLAUNCH_CHECK();
         richards_residual<<<nbN, kRBlock, 0, stream>>>((int)N, irp, ifc, fa, fb, faol, rc_Kh, lv[0].dir, rc_psi,
                                                        rc_z, rc_Q, shift_dev, psi_old, rc_R, rc_part);
@@ -470,8 +481,8 @@ int GeneralSolver::richards_nonlinear(const double *shift_dev, const double *psi
     }
     iters = it;
     relres = scale > 0 ? rn / scale : 0.0;
-    kr_faces<<<nbF, kRBlock, 0, stream>>>((int)F, fa, fb, faol, rc_Ks, rc_al, rc_N, rc_psi, rc_z, rc_Kh, rc_na,
-                                          rc_nb);
+    kr_faces<true><<<nbF, kRBlock, 0, stream>>>((int)F, fa, fb, faol, rc_Ks, rc_al, rc_N, rc_psi, rc_z, rc_Kh, rc_na,
+                                                rc_nb);
     GLAUNCH_CHECK();
     rck(cudaStreamSynchronize(stream), "sync");
     if (!std::isfinite(rn)) return DPF_NAN;
@@ -502,7 +513,7 @@ int GeneralSolver::richards_gmres(const double *rhs_dev, double *x_dev, const do
         richards_adjoint_rhs<<<nbN, kRBlock, 0, stream>>>((int)N, irp, ifc, fa, fb, rc_na, rc_nb, lv[0].dir, rc_zero,
                                                           v, rc_R);
         GLAUNCH_CHECK();
-        const int src = richards_spd_solve(rc_R, out, shift_dev);
+        const int src = richards_spd_solve(rc_R, out, shift_dev, true);
         if (src != DPF_OK && src != DPF_NOT_CONVERGED) return src;
         axpby(1.0, v, -1.0, out);
         return DPF_OK;
@@ -614,8 +625,8 @@ int GeneralSolver::richards_adjoint(const double *delta_in, double tol, int maxi
                                                      lv[0].dir, rc_mu, dKs ? rc_gK : nullptr,
                                                      dalphas ? rc_ga : nullptr, dNs ? rc_gN : nullptr, 0);
     GLAUNCH_CHECK();
-    richards_cell_grads<<<nbN, kRBlock, 0, stream>>>((int)N, irp, ifc, fa, fb, faol, rc_Ks, rc_al, rc_N, rc_psi,
-                                                     rc_z, lv[0].dir, rc_mu, rc_delta, dQs ? rc_d : nullptr,
+    richards_cell_grads<<<nbN, kRBlock, 0, stream>>>((int)N, irp, ifc, fa, fb, faol, rc_Kh, rc_na, rc_nb,
+                                                     lv[0].dir, rc_mu, rc_delta, dQs ? rc_d : nullptr,
                                                      ddpsi ? rc_R : nullptr, 0);
     GLAUNCH_CHECK();
     rcopy_out(dKs, rc_gK, F, stream);
@@ -715,8 +726,8 @@ int GeneralSolver::richards_transient_adjoint(long long nobs, const int64_t *obs
     for (int n = nsteps; n >= 1; n--) {
         const double *psi_n = rt_states + (size_t)n * N;
         rck(cudaMemcpyAsync(rc_psi, psi_n, N * sizeof(double), cudaMemcpyDeviceToDevice, stream), "state");
-        kr_faces<<<nbF, kRBlock, 0, stream>>>((int)F, fa, fb, faol, rc_Ks, rc_al, rc_N, rc_psi, rc_z, rc_Kh, rc_na,
-                                              rc_nb);
+        kr_faces<true><<<nbF, kRBlock, 0, stream>>>((int)F, fa, fb, faol, rc_Ks, rc_al, rc_N, rc_psi, rc_z, rc_Kh,
+                                                    rc_na, rc_nb);
         GLAUNCH_CHECK();
         // seed = dJ/dpsi^n
         if (n == nsteps && d_gT)
@@ -741,8 +752,8 @@ int GeneralSolver::richards_transient_adjoint(long long nobs, const int64_t *obs
                                                          lv[0].dir, lam, dKs ? rc_gK : nullptr,
                                                          dalphas ? rc_ga : nullptr, dNs ? rc_gN : nullptr, acc);
         GLAUNCH_CHECK();
-        richards_cell_grads<<<nbN, kRBlock, 0, stream>>>((int)N, irp, ifc, fa, fb, faol, rc_Ks, rc_al, rc_N, rc_psi,
-                                                         rc_z, lv[0].dir, lam, seed, dQs ? rt_gQ : nullptr,
+        richards_cell_grads<<<nbN, kRBlock, 0, stream>>>((int)N, irp, ifc, fa, fb, faol, rc_Kh, rc_na, rc_nb,
+                                                         lv[0].dir, lam, seed, dQs ? rt_gQ : nullptr,
                                                          ddpsi ? rt_gD : nullptr, acc);
         GLAUNCH_CHECK();
         rck(cudaMemcpyAsync(lam_hold, lam, N * sizeof(double), cudaMemcpyDeviceToDevice, stream), "lam");

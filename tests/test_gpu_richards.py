@@ -94,3 +94,23 @@ def test_thiem_richards_matches_groundwater(gpu_lib):
     dd_r = t["steadyhead"] - psi[t["good"]]
     assert np.linalg.norm(dd_r - dd_gw) <= 1e-8 * np.linalg.norm(dd_gw)
     assert np.linalg.norm(t["thiem"] - dd_r) <= 1e-1 * max(np.linalg.norm(t["thiem"]), np.linalg.norm(dd_r))
+
+
+@pytest.mark.parametrize("nvg,psi_top,zero_alpha", [(1.12, -1.5, False), (2.0, -1.0, False), (2.7, -0.8, True)])
+@pytest.mark.parametrize("solver", ["cg", "cholesky"])
+def test_van_genuchten_range(gpu_lib, nvg, psi_top, zero_alpha, solver):
+    """Exponents from 1.12 to 2.75, faces with alpha = 0 (kr = 1 everywhere), both solvers."""
+    pkg = gpu_lib
+    c = richards_case(pkg, ns=(7, 5, 4), psi_top=psi_top, nvg=nvg, seed=3)
+    if zero_alpha:
+        c["alphas"][::3] = 0.0
+    psi_or = ro.steady(c["psi0"], c["Ks"], c["nb"], c["aol"], c["dn"], c["dpsi"], c["z"], c["alphas"], c["Ns"],
+                       c["Qs"], tol=1e-14)
+    w = np.random.default_rng(5).standard_normal(c["N"])
+    g_or = ro.pullback(psi_or, w, *oracle_args(c))
+    P = pkg.GroundwaterProblem(c["nb"], c["aol"], c["dn"], N=c["N"], general=True, solver=solver, reltol=1e-12)
+    psi = P.richards_steady(c["psi0"], c["Ks"], c["dpsi"], c["z"], c["alphas"], c["Ns"], c["Qs"], tol=1e-12)
+    assert rel(psi, psi_or) < 1e-9
+    g = P.richards_adjoint(w, tol=1e-12)
+    for got, want, name in zip(g, g_or, ("dKs", "ddirichletpsis", "dalphas", "dNs", "dQs")):
+        assert rel(got, want) < 1e-7, name
