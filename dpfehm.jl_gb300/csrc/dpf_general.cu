@@ -57,8 +57,7 @@ __device__ __forceinline__ double g_face_k(const double *Ks, const double *kc, i
 // ------------------------------------------------------------ set-up kernels
 __global__ void kg_cell_k(int n, const double *__restrict__ logK, int kind, double *__restrict__ kc) {
     GSTRIDE(i, n) {
-        double v = logK[i];
-        kc[i] = exp(kind == DPF_MEAN_GEOMETRIC ? 0.5 * v : v);
+        kc[i] = cell_k(logK[i], kind);
     }
 }
 
@@ -75,10 +74,9 @@ __global__ void kg_vjp(int n, const int *__restrict__ irp, const int *__restrict
         double ki = kc[i], acc = 0.0;
         for (int k = irp[i]; k < irp[i + 1]; k++) {
             int f = ifc[k];
-            double K = face_mean_k(ki, kc[other_end(fa, fb, f, i)], kind);
-            acc += face_mean_dlogk(K, ki, kind) * dKs[f];
+            acc = fma(dlogk_weight(ki, kc[other_end(fa, fb, f, i)], kind), dKs[f], acc);
         }
-        g[i] = acc;
+        g[i] = dlogk_scale(ki, kind) * acc;
     }
 }
 
@@ -593,10 +591,9 @@ __global__ void kg_grad_logk(int n, const int *__restrict__ irp, const int *__re
             int f = ifc[k];
             int j = other_end(fa, fb, f, i);
             double dK = -faol[f] * (hi - h[j]) * (li - lam[j]);
-            double K = face_mean_k(ki, kc[j], kind);
-            acc += face_mean_dlogk(K, ki, kind) * dK;
+            acc = fma(dlogk_weight(ki, kc[j], kind), dK, acc);
         }
-        g[i] = acc;
+        g[i] = dlogk_scale(ki, kind) * acc;
     }
 }
 

@@ -29,6 +29,7 @@
 #include <string>
 
 #include "dpf_internal.h"
+#include "dpf_means.cuh"
 
 namespace {
 
@@ -54,8 +55,7 @@ __device__ __forceinline__ long long na_face_index(int nx, int ny, int nz, int i
 __global__ void k_na_cell(long long n, const double *__restrict__ logK, int kind, double *__restrict__ kc) {
     long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
     if (i >= n) return;
-    double v = logK[i];
-    kc[i] = exp(kind == DPF_MEAN_GEOMETRIC ? 0.5 * v : v);
+    kc[i] = dpf::cell_k(logK[i], kind);
 }
 
 __global__ void k_na_faces(int nx, int ny, int nz, unsigned mag_nz, int sh_nz, unsigned mag_ny, int sh_ny,
@@ -74,9 +74,7 @@ __global__ void k_na_faces(int nx, int ny, int nz, unsigned mag_nz, int sh_nz, u
     const double ka = kc[li];
     for (int d = 0; d < 3; d++) {
         if (co[d] + 1 >= nn[d]) continue;
-        double kb = kc[li + st[d]];
-        double K = kind == DPF_MEAN_GEOMETRIC ? ka * kb : 2.0 * ka * kb / (ka + kb);
-        Ks[na_face_index(nx, ny, nz, ix, iy, iz, d)] = K;
+        Ks[na_face_index(nx, ny, nz, ix, iy, iz, d)] = dpf::face_mean_k(ka, kc[li + st[d]], kind);
     }
 }
 

@@ -1025,7 +1025,9 @@ __global__ void k_grad_faces(const LevelDesc *__restrict__ desc, const int4 *__r
 }
 
 // dlogK_i = sum over the faces of i of dK_f/dlogK_i * dKs_f, with dKs_f formed on the fly
-// from h and lambda; K_f and its derivative come from the per-cell values kc.
+// from h and lambda and dK_f/dlogK_i = scale(kc_i) weight(kc_i, kc_j), the scale taken out of the sum.
+// FP64 instructions bound it: 4 per face of a cell (geometric) or 12 (harmonic; with two divisions per
+// face, 30, the 7.1M cells of a batch of uneven grids took 1950 us, 1133 us now).
 __global__ void k_grad_logk(const LevelDesc *__restrict__ desc, const int4 *__restrict__ bmap,
                             const ProbParam *__restrict__ prm, const double *__restrict__ kc, int kind,
                             const double *__restrict__ h, const double *__restrict__ lam, double *__restrict__ g) {
@@ -1041,38 +1043,20 @@ __global__ void k_grad_logk(const LevelDesc *__restrict__ desc, const int4 *__re
         const int nn[3] = {L.nx, L.ny, L.nz};
         const double hi = h[c.i], li = lam[c.i], ki = kc[c.i];
         double acc = 0.0;
-        if (kind == DPF_MEAN_GEOMETRIC) {
-            // dK_f/dlogK_i = K_f / 2 = kc_i kc_j / 2: per direction sum kc_j (h_i-h_j)(l_i-l_j),
-            // then scale by -aol kc_i / 2 (4 FP64 operations per face)
-    #pragma unroll
-            for (int d = 0; d < 3; d++) {
-                double sd = 0.0;
-                if (co[d] + 1 < nn[d]) {
-                    const long long j = c.i + st3[d];
-                    sd = fma(kc[j], (hi - h[j]) * (li - lam[j]), sd);
-                }
-                if (co[d] > 0) {
-                    const long long j = c.i - st3[d];
-                    sd = fma(kc[j], (hi - h[j]) * (li - lam[j]), sd);
-                }
-                acc = fma(-0.5 * P.aol[d] * ki, sd, acc);
-            }
-            g[c.i] = acc;
-            continue;
-        }
     #pragma unroll
         for (int d = 0; d < 3; d++) {
-    #pragma unroll
-            for (int s = -1; s <= 1; s += 2) {
-                bool ok = s > 0 ? co[d] + 1 < nn[d] : co[d] > 0;
-                if (!ok) continue;
-                long long j = c.i + s * st3[d];
-                double dK = -P.aol[d] * (hi - h[j]) * (li - lam[j]);
-                double K = face_mean_k(ki, kc[j], kind);
-                acc += face_mean_dlogk(K, ki, kind) * dK;
+            double sd = 0.0;
+            if (co[d] + 1 < nn[d]) {
+                const long long j = c.i + st3[d];
+                sd = fma(dlogk_weight(ki, kc[j], kind), (hi - h[j]) * (li - lam[j]), sd);
             }
+            if (co[d] > 0) {
+                const long long j = c.i - st3[d];
+                sd = fma(dlogk_weight(ki, kc[j], kind), (hi - h[j]) * (li - lam[j]), sd);
+            }
+            acc = fma(-P.aol[d], sd, acc);
         }
-        g[c.i] = acc;
+        g[c.i] = dlogk_scale(ki, kind) * acc;
     }
 }
 
@@ -1134,18 +1118,15 @@ __global__ void k_grad_logk_df(const LevelDesc *__restrict__ desc, const int4 *_
     }
 }
 
-// per-cell values for the face means: exp(logK / 2) (geometric) or exp(logK) (harmonic)
+// per-cell values for the face means; FP64 arithmetic bounds it (8M cells: 249 us with the library's
+// exponential, about 15 FP64 instructions; 156 us with the 8 of exp64)
 __global__ void k_cell_k(const LevelDesc *__restrict__ desc, const int4 *__restrict__ bmap,
                          const double *__restrict__ logK, int kind, double *__restrict__ kc) {
     pdl_enter();
     int4 bm = bmap[blockIdx.x];
     const LevelDesc L = desc[bm.x];
-    for (int li_ = bm.y * kBlock + (int)threadIdx.x; li_ < (int)L.n; li_ += bm.z * kBlock) {
-        Cell c;
-        cell_at(L, li_, c);
-        double v = logK[c.i];
-        kc[c.i] = exp(kind == DPF_MEAN_GEOMETRIC ? 0.5 * v : v);
-    }
+    for (int li_ = bm.y * kBlock + (int)threadIdx.x; li_ < (int)L.n; li_ += bm.z * kBlock)
+        kc[L.off + li_] = cell_k(logK[L.off + li_], kind);
 }
 
 // the smoothers' diagonals of a level: FP64 levels the diagonal and its inverse (they multiply
@@ -1208,55 +1189,81 @@ __global__ void k_grad_dh_q(const LevelDesc *__restrict__ desc, const int4 *__re
     }
 }
 
-// Ks in the reference face order from the per-cell values kc
-__global__ void k_logk_to_faces(const LevelDesc *__restrict__ desc, const int4 *__restrict__ bmap,
-                                const ProbParam *__restrict__ prm, const double *__restrict__ kc, int kind,
-                                double *__restrict__ Ks) {
+// Ks in the reference face order from the per-cell values kc. The faces of consecutive cells are consecutive,
+// two or three per cell: a warp gathers those of its 32 cells in shared memory and writes them as whole lines
+// (stored from the cells' threads they touched every sector three times, and the L2's write rate bound the
+// kernel). Memory-bound with 32 bytes per cell, near the 3 FP64 products: 8M cells 81 us -> 58 us.
+template <int kKind>
+__global__ void __launch_bounds__(kBlock) k_logk_to_faces(const LevelDesc *__restrict__ desc, const int4 *__restrict__ bmap,
+                                                          const ProbParam *__restrict__ prm,
+                                                          const double *__restrict__ kc, double *__restrict__ Ks) {
+    __shared__ double buf[kBlock * 3];
     pdl_enter();
-    int4 bm = bmap[blockIdx.x];
+    const int4 bm = bmap[blockIdx.x];
     const LevelDesc L = desc[bm.x];
-    for (int li_ = bm.y * kBlock + (int)threadIdx.x; li_ < (int)L.n; li_ += bm.z * kBlock) {
+    double *const Kp = Ks + prm[bm.x].face_off;
+    const long long sy = L.nz, sx = (long long)L.ny * L.nz;
+    const int lane = threadIdx.x & 31;
+    double *const wb = buf + (threadIdx.x - lane) * 3;
+    for (int li_ = bm.y * kBlock + (int)threadIdx.x; li_ - lane < (int)L.n; li_ += bm.z * kBlock) {
+        const bool on = li_ < (int)L.n;
         Cell c;
-        cell_at(L, li_, c);
-        const ProbParam P = prm[bm.x];
-        const long long st3[3] = {(long long)L.ny * L.nz, (long long)L.nz, 1};
-        const int co[3] = {c.ix, c.iy, c.iz};
-        const int nn[3] = {L.nx, L.ny, L.nz};
-        for (int d = 0; d < 3; d++)
-            if (co[d] + 1 < nn[d])
-                Ks[P.face_off + regular_face_index(L.nx, L.ny, L.nz, c.ix, c.iy, c.iz, d)] =
-                    face_mean_k(kc[c.i], kc[c.i + st3[d]], kind);
+        cell_at(L, on ? li_ : (int)L.n - 1, c);
+        const int ex = c.ix + 1 < L.nx, ey = c.iy + 1 < L.ny, ez = c.iz + 1 < L.nz;
+        const double ki = kc[c.i], kx = ex ? kc[c.i + sx] : 0.0, ky = ey ? kc[c.i + sy] : 0.0,
+                     kz = ez ? kc[c.i + 1] : 0.0;
+        const long long f = regular_face_index(L.nx, L.ny, L.nz, c.ix, c.iy, c.iz, 0);
+        const long long f0 = __shfl_sync(0xffffffffu, f, 0);
+        const int at = (int)(f - f0), total = __shfl_sync(0xffffffffu, at + ex + ey + ez, 31);
+        if (on) {
+            if (ex) wb[at] = face_mean_k(ki, kx, kKind);
+            if (ey) wb[at + ex] = face_mean_k(ki, ky, kKind);
+            if (ez) wb[at + ex + ey] = face_mean_k(ki, kz, kKind);
+        }
+        __syncwarp();
+    #pragma unroll
+        for (int k = 0; k < 3; k++)
+            if (lane + 32 * k < total) Kp[f0 + lane + 32 * k] = wb[lane + 32 * k];
+        __syncwarp();
     }
 }
 
-// dlogK from dKs (gather over the six faces of each cell)
+// dlogK from dKs (gather over the six faces of each cell), dK_f/dlogK_i as in k_grad_logk. The faces that a
+// cell owns are consecutive; those owned by its -y and -z neighbours follow from the cell's own first face.
+// FP64-bound (8 instructions per cell, geometric): 123 us for 8M cells, 275 us with the derivative formed
+// per face and the index per face.
+template <int kKind>
 __global__ void k_logk_vjp(const LevelDesc *__restrict__ desc, const int4 *__restrict__ bmap,
-                           const ProbParam *__restrict__ prm, const double *__restrict__ kc, int kind,
+                           const ProbParam *__restrict__ prm, const double *__restrict__ kc,
                            const double *__restrict__ dKs, double *__restrict__ g) {
     pdl_enter();
     int4 bm = bmap[blockIdx.x];
     const LevelDesc L = desc[bm.x];
+    const double *const dk = dKs + prm[bm.x].face_off;
+    const long long sy = L.nz, sx = (long long)L.ny * L.nz;
     for (int li_ = bm.y * kBlock + (int)threadIdx.x; li_ < (int)L.n; li_ += bm.z * kBlock) {
         Cell c;
         cell_at(L, li_, c);
-        const ProbParam P = prm[bm.x];
-        const long long st3[3] = {(long long)L.ny * L.nz, (long long)L.nz, 1};
-        const int co[3] = {c.ix, c.iy, c.iz};
-        const int nn[3] = {L.nx, L.ny, L.nz};
+        const int ex = c.ix + 1 < L.nx, ey = c.iy + 1 < L.ny, ez = c.iz + 1 < L.nz;
+        const long long f = regular_face_index(L.nx, L.ny, L.nz, c.ix, c.iy, c.iz, 0);
         const double ki = kc[c.i];
+        // the line below: (ex + 1 + 1) faces per cell, the last cell of a line one less
+        const long long fy = f - (long long)(ex * L.nz + 2 * L.nz - 1) + c.iz * (1 - ey) + ex;
+        const long long fx = regular_face_index(L.nx, L.ny, L.nz, c.ix - 1, c.iy, c.iz, 0);
+        const bool on[6] = {ex != 0, ey != 0, ez != 0, c.ix > 0, c.iy > 0, c.iz > 0};
+        const long long at[6] = {f, f + ex, f + ex + ey, fx, fy, f - 1};
+        const long long st[6] = {sx, sy, 1, -sx, -sy, -1};
+        double kj[6], dj[6];
+    #pragma unroll
+        for (int k = 0; k < 6; k++) {
+            kj[k] = on[k] ? kc[c.i + st[k]] : 0.0;
+            dj[k] = on[k] ? dk[at[k]] : 0.0;
+        }
         double acc = 0.0;
-        for (int d = 0; d < 3; d++)
-            for (int s = -1; s <= 1; s += 2) {
-                bool ok = s > 0 ? co[d] + 1 < nn[d] : co[d] > 0;
-                if (!ok) continue;
-                long long j = c.i + s * st3[d];
-                int ax = c.ix, ay = c.iy, az = c.iz;
-                if (s < 0) { if (d == 0) ax--; else if (d == 1) ay--; else az--; }
-                long long f = P.face_off + regular_face_index(L.nx, L.ny, L.nz, ax, ay, az, d);
-                double K = face_mean_k(ki, kc[j], kind);
-                acc += face_mean_dlogk(K, ki, kind) * dKs[f];
-            }
-        g[c.i] = acc;
+    #pragma unroll
+        for (int k = 0; k < 6; k++)
+            if (on[k]) acc = fma(dlogk_weight(ki, kj[k], kKind), dj[k], acc);
+        g[c.i] = dlogk_scale(ki, kKind) * acc;
     }
 }
 
@@ -2970,7 +2977,8 @@ void StructBatch::logk_to_faces(const double *logK, int kind, double *Ks) {
     cell_k(logK, kind, aux_kc);
     {
         KTimer _kt(this, kname("k_logk_to_faces", 0, false), L0.all_cells);
-        k_logk_to_faces<<<nb_of(L0.all), kBlock, 0, stream>>>(L0.d_desc, L0.all.d_map, d_prm, aux_kc, kind, Ks);
+        auto kern = kind == DPF_MEAN_GEOMETRIC ? k_logk_to_faces<DPF_MEAN_GEOMETRIC> : k_logk_to_faces<DPF_MEAN_HARMONIC>;
+        kern<<<nb_of(L0.all), kBlock, 0, stream>>>(L0.d_desc, L0.all.d_map, d_prm, aux_kc, Ks);
     }
     LAUNCH_CHECK();
 }
@@ -2980,7 +2988,8 @@ void StructBatch::logk_vjp(const double *logK, int kind, const double *dKs, doub
     cell_k(logK, kind, aux_kc);
     {
         KTimer _kt(this, kname("k_logk_vjp", 0, false), L0.all_cells);
-        k_logk_vjp<<<nb_of(L0.all), kBlock, 0, stream>>>(L0.d_desc, L0.all.d_map, d_prm, aux_kc, kind, dKs, g);
+        auto kern = kind == DPF_MEAN_GEOMETRIC ? k_logk_vjp<DPF_MEAN_GEOMETRIC> : k_logk_vjp<DPF_MEAN_HARMONIC>;
+        kern<<<nb_of(L0.all), kBlock, 0, stream>>>(L0.d_desc, L0.all.d_map, d_prm, aux_kc, dKs, g);
     }
     LAUNCH_CHECK();
 }

@@ -8,6 +8,7 @@
 #pragma once
 #include "dpf_check.cuh"
 #include "dpf_internal.h"
+#include "dpf_means.cuh"
 
 namespace dpf {
 
@@ -435,20 +436,6 @@ __device__ __forceinline__ bool split48(double v, float &hi, float &lo, double &
     lo = __uint_as_float(__float_as_uint(lo_mag) | sign);
     v48 = __longlong_as_double((long long)u);
     return true;
-}
-
-// Face conductances from cell values kc, computed once per cell by k_cell_k
-// (GB300 has little FP64 throughput, so exp runs once per cell, not once per face):
-//   geometric  kc = exp(logK / 2):  K_f = exp((logK_a + logK_b)/2) = kc_a kc_b
-//   harmonic   kc = exp(logK):      K_f = 2 / (1/K_a + 1/K_b) = 2 kc_a kc_b / (kc_a + kc_b)
-__device__ __forceinline__ double face_mean_k(double ka, double kb, int kind) {
-    if (kind == DPF_MEAN_GEOMETRIC) return ka * kb;
-    return 2.0 * ka * kb / (ka + kb);
-}
-// dK_f / dlogK_a:  geometric K_f / 2;  harmonic K_f^2 / (2 K_a)
-__device__ __forceinline__ double face_mean_dlogk(double Kf, double ka, int kind) {
-    if (kind == DPF_MEAN_GEOMETRIC) return 0.5 * Kf;
-    return 0.5 * Kf * Kf / ka;
 }
 
 }  // namespace dpf

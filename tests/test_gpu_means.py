@@ -1,0 +1,58 @@
+"""Face conductances from logK and their pullback against extended precision: the table-driven exponential
+and the division of dpf_means.cuh over their whole range. Bounds: an exponential is within 0.54 ulp, a product,
+sum or quotient within half an ulp."""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+EPS = 2.0 ** -52
+
+
+def _case(pkg, ns, lim, seed=0):
+    coords, nb, aol, _ = pkg.regulargrid3d((0.0, 0.0, 0.0), (1.0, 1.0, 1.0), ns)
+    rng = np.random.default_rng(seed)
+    logK = rng.uniform(-lim, lim, coords.shape[1])
+    return nb, aol, logK, rng.standard_normal(len(nb))
+
+
+@pytest.mark.parametrize("general", [False, True])
+@pytest.mark.parametrize("mean", ["geometric", "harmonic"])
+@pytest.mark.parametrize("ns,lim", [((33, 17, 9), 0.01), ((33, 17, 9), 12.0), ((40, 1, 7), 160.0), ((2, 50, 1), 690.0)])
+def test_means_and_pullback(gpu_lib, ns, lim, mean, general):
+    nb, aol, logK, dKs = _case(gpu_lib, ns, lim)
+    P = gpu_lib.GroundwaterProblem(nb, aol, np.array([0]), N=len(logK), general=general)
+    assert P.structured != general
+    a, b = nb[:, 0], nb[:, 1]
+    with np.errstate(all="ignore"):
+        k = np.exp(logK.astype(np.longdouble) / (2 if mean == "geometric" else 1))
+        s = 1.0 if mean == "geometric" else k[a] + k[b]
+        K = k[a] * k[b] if mean == "geometric" else 2 * k[a] * k[b] / s
+        ga, gb = (K / 2, K / 2) if mean == "geometric" else (2 * k[a] * (k[b] / s) ** 2, 2 * k[b] * (k[a] / s) ** 2)
+    got = P.logk_to_faces(logK, mean)
+    assert np.all(np.abs(got - K) <= 2.1 * EPS * K + 5e-324)
+    g = P.logk_to_faces_vjp(logK, dKs, mean)
+    want, size = np.zeros(len(logK), np.longdouble), np.zeros(len(logK), np.longdouble)
+    for i, w in ((a, ga * dKs), (b, gb * dKs)):
+        np.add.at(want, i, w)
+        np.add.at(size, i, np.abs(w))
+    assert np.all(np.abs(g - want) <= 12 * EPS * size + 1e-300)
+
+
+@pytest.mark.parametrize("general", [False, True])
+def test_limits(gpu_lib, general):
+    """Cell values beyond the reduced range: overflow, underflow, subnormals, infinities and NaN."""
+    v = np.array([0.0, -0.0, 699.99, 700.0, 709.7, 710.0, -699.99, -700.0, -740.0, -746.0, np.inf, -np.inf, np.nan,
+                  1399.9, 1400.0, 1419.0, -1399.9, -1400.0, 1e300, -1e300, 5e-324])
+    n = len(v)
+    nb = np.stack([np.arange(n), np.arange(n) + n], 1)   # each value beside a 1: K = exp(v / 2), 2 K / (1 + K)
+    logK = np.concatenate([v, np.zeros(n)])
+    if not general:
+        coords, nb, aol, _ = gpu_lib.regulargrid3d((0.0, 0.0, 0.0), (1.0, 1.0, 1.0), (2, n, 1))
+        faces = np.nonzero(nb[:, 1] - nb[:, 0] == n)[0]
+    else:
+        aol, faces = np.ones(n), np.arange(n)
+    P = gpu_lib.GroundwaterProblem(nb, aol, np.array([0]), N=2 * n, general=general)
+    with np.errstate(all="ignore"):
+        np.testing.assert_allclose(P.logk_to_faces(logK, "geometric")[faces], np.exp(v / 2), rtol=4 * EPS, atol=1e-323)
+        k = np.exp(v)
+        np.testing.assert_allclose(P.logk_to_faces(logK, "harmonic")[faces], 2 * (k / (k + 1)), rtol=6 * EPS, atol=1e-323)
