@@ -261,6 +261,20 @@ const T *stage_in(dpf_problem *P, const T *src, size_t n, T *dst) {
     return dst;
 }
 
+// Whether a kernel of this handle can read n elements at src where they are: memory of its device, aligned,
+// and apart from the m elements at out that the call writes. (Eight 1M-cell grids: copying logK and dKs first,
+// and allocating and freeing a buffer for dKs, was 0.4 of the 0.92 ms of a pair of calls.)
+bool readable_in_place(const dpf_problem *P, const double *src, size_t n, const double *out, size_t m) {
+    cudaPointerAttributes a;
+    if (cudaPointerGetAttributes(&a, src) != cudaSuccess) {
+        cudaGetLastError();
+        return false;
+    }
+    const uintptr_t s = (uintptr_t)src, o = (uintptr_t)out;
+    return a.type == cudaMemoryTypeDevice && a.device == P->device && s % sizeof(double) == 0 &&
+           (s + n * sizeof(double) <= o || o + m * sizeof(double) <= s);
+}
+
 template <typename T>
 void stage_out(dpf_problem *P, T *dst, const T *src, size_t n) {
     if (!dst) return;
@@ -831,9 +845,9 @@ int dpf_logk_to_faces(dpf_problem *P, const double *logK, int kind, double *Ks) 
         if (kind != DPF_MEAN_GEOMETRIC && kind != DPF_MEAN_HARMONIC) throw BadInput("unknown mean kind");
         if (P->gs) return gs_status(P, P->gs->logk_to_faces(logK, kind, Ks));
         StructBatch &S = *P->sb;
-        stage_in(P, logK, S.N, S.in_logK);
+        if (!readable_in_place(P, logK, S.N, Ks, S.F)) logK = stage_in(P, logK, S.N, S.in_logK);
         double *tmp = is_device_ptr(Ks) ? Ks : S.in_Ks;
-        S.logk_to_faces(S.in_logK, kind, tmp);
+        S.logk_to_faces(logK, kind, tmp);
         if (tmp != Ks) stage_out(P, Ks, tmp, S.F);
         return DPF_OK;
     });
@@ -845,14 +859,17 @@ int dpf_logk_to_faces_vjp(dpf_problem *P, const double *logK, int kind, const do
         if (kind != DPF_MEAN_GEOMETRIC && kind != DPF_MEAN_HARMONIC) throw BadInput("unknown mean kind");
         if (P->gs) return gs_status(P, P->gs->logk_vjp(logK, kind, dKs, dlogK));
         StructBatch &S = *P->sb;
-        stage_in(P, logK, S.N, S.in_logK);
-        double *dk = scratch<double>(P, S.F);
-        stage_in(P, dKs, S.F, dk);
+        if (!readable_in_place(P, logK, S.N, dlogK, S.N)) logK = stage_in(P, logK, S.N, S.in_logK);
+        double *dk = nullptr;
+        if (!readable_in_place(P, dKs, S.F, dlogK, S.N)) {
+            dk = scratch<double>(P, S.F);
+            dKs = stage_in(P, dKs, S.F, dk);
+        }
         double *tmp = is_device_ptr(dlogK) ? dlogK : S.r64;
-        S.logk_vjp(S.in_logK, kind, dk, tmp);
+        S.logk_vjp(logK, kind, dKs, tmp);
         if (tmp != dlogK) stage_out(P, dlogK, tmp, S.N);
         ck(cudaStreamSynchronize(P->stream), "sync");
-        release(P, dk);
+        if (dk) release(P, dk);
         return DPF_OK;
     });
 }

@@ -56,3 +56,40 @@ def test_limits(gpu_lib, general):
         np.testing.assert_allclose(P.logk_to_faces(logK, "geometric")[faces], np.exp(v / 2), rtol=4 * EPS, atol=1e-323)
         k = np.exp(v)
         np.testing.assert_allclose(P.logk_to_faces(logK, "harmonic")[faces], 2 * (k / (k + 1)), rtol=6 * EPS, atol=1e-323)
+
+
+@pytest.mark.parametrize("where", ["host", "device", "overlap", "offset"])
+def test_arrays_in_place(gpu_lib, where):
+    """Inputs on the host, on the device, overlapping the output and at an address between two doubles: the same."""
+    import ctypes
+    import torch
+    nb, aol, logK, dKs = _case(gpu_lib, (9, 8, 7), 3.0)
+    n, F = len(logK), len(nb)
+    P = gpu_lib.GroundwaterProblem(nb, aol, np.array([0]), N=n)
+    want_K, want_g = P.logk_to_faces(logK), P.logk_to_faces_vjp(logK, dKs)
+    if where == "host":
+        got_K, got_g = P.logk_to_faces(logK.copy()), P.logk_to_faces_vjp(logK.copy(), dKs.copy())
+    else:
+        raw = torch.zeros(8 * (3 * F + 2 * n) + 64, dtype=torch.uint8, device="cuda")
+        off = 4 if where == "offset" else 0
+
+        def put(at, v):
+            raw[at:at + 8 * len(v)] = torch.from_numpy(v.view(np.uint8).copy()).cuda()
+            torch.cuda.synchronize()
+            return raw.data_ptr() + at
+
+        def get(at, m):
+            torch.cuda.synchronize()
+            return raw[at:at + 8 * m].cpu().numpy().view(np.float64)
+
+        lk, dk, K = off, 8 * n + 16 + off, 8 * (n + F) + 32
+        g = 8 * (n + 2 * F) + 48
+        if where == "overlap":
+            K, g = lk, dk + 8 * 5
+        _f = lambda name, *a: gpu_lib._check(P._lib, P._h, getattr(P._lib, name)(P._h, *a))
+        _f("dpf_logk_to_faces", ctypes.c_void_p(put(lk, logK)), 0, ctypes.c_void_p(raw.data_ptr() + K))
+        got_K = get(K, F)
+        _f("dpf_logk_to_faces_vjp", ctypes.c_void_p(put(lk, logK)), 0, ctypes.c_void_p(put(dk, dKs)),
+           ctypes.c_void_p(raw.data_ptr() + g))
+        got_g = get(g, n)
+    assert np.array_equal(got_K, want_K) and np.array_equal(got_g, want_g)
