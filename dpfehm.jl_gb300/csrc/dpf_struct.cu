@@ -1423,11 +1423,18 @@ static BlockMap build_map(const std::vector<LevelDesc> &desc, const std::vector<
 // Plane-marching work of a level. Per smoothed problem the grid is cut into slabs of whole
 // rows (plane_rows: up to `cells` cells, so a slab is contiguous in every array), and the
 // planes of all slabs of all problems form one sequence of plane pairs (the restriction sums
-// pairs of planes) weighted by their cells. The sequence is cut into contiguous runs of about
+// pairs of planes) weighted by the time they take. The sequence is cut into contiguous runs of about
 // equal weight, one per block (SMs x blocks_per_sm blocks, fewer on small levels), so
 // every block of a launch gets the same work whatever the batch's sizes; a run that crosses a
 // slab boundary becomes several items, which the block marches through one after another.
 // Items start on even planes and end on one, or on the grid's last plane.
+// The weight of a plane is its cells plus kPlaneCost: a plane's waits, barriers and shared-memory
+// latency take about the time of 1500 cells however few it has, so blocks that were given the planes
+// of the batch's small grids by their cells alone finished last (24 grids of 12.5k to 800k cells: a
+// smoothing step 75 us, 48 us so; the solve and gradient 21.3 -> 17.2 ms; 700 gave 17.9, 2500 17.4).
+// Starting a slab (a block barrier, the reduction, a plane of halo, the ring running empty) costs two
+// planes more (64 grids of 100k cells: 14.3 -> 13.9 ms; half as much 14.1, none 14.3).
+constexpr int kPlaneCost = 1500, kSlabCost = 3000;
 void StructBatch::build_plane_items(PlaneItems &P, const Level &L, const std::vector<int> &take, int sms,
                                     int cells, int blocks_per_sm,
                                     const std::vector<std::vector<std::array<int, 3>>> *shapes, int l) {
@@ -1437,13 +1444,8 @@ void StructBatch::build_plane_items(PlaneItems &P, const Level &L, const std::ve
     // per SM, and the FP64 smoothers are faster as grid-stride kernels
     if (cells <= 0 || !mixed) return;
     long long total = 0;
-    for (int p = 0; p < nprob; p++) {
-        if (!take[p]) continue;
-        const LevelDesc &D = L.h_desc[p];
-        if (D.nz > cells) return;  // a row must fit a slab
-        total += D.n;
-    }
-    if (total == 0) return;
+    for (int p = 0; p < nprob; p++)
+        if (take[p] && L.h_desc[p].nz > cells) return;  // a row must fit a slab
     // the units: plane pairs of every slab, in problem, slab, plane order
     struct Unit {
         int p, y0, x0, x1;
@@ -1458,7 +1460,8 @@ void StructBatch::build_plane_items(PlaneItems &P, const Level &L, const std::ve
             const long long rc = (long long)std::min(Ty, D.ny - y0) * D.nz;
             for (int x0 = 0; x0 < D.nx; x0 += 2) {
                 const int x1 = std::min(x0 + 2, D.nx);
-                units.push_back(Unit{p, y0, x0, x1, rc * (x1 - x0)});
+                units.push_back(Unit{p, y0, x0, x1, (rc + kPlaneCost) * (x1 - x0) + (x0 == 0 ? kSlabCost : 0)});
+                total += units.back().w;
             }
         }
         P.halo = std::max(P.halo, (Ty + 2) * D.nz);
@@ -1472,6 +1475,7 @@ void StructBatch::build_plane_items(PlaneItems &P, const Level &L, const std::ve
             P.coarse2 = std::max(P.coarse2, ((Ty + 4) / 2 + 2) * cnz);
         }
     }
+    if (total == 0) return;
     // on the finest level at least 4 plane pairs per block where the level allows: every run also
     // stages the plane on each side of it, which for shorter runs costs more bandwidth than the
     // parallelism gains; the coarser levels are latency-bound and take as many blocks as they can
