@@ -851,8 +851,10 @@ GeneralSolver::GeneralSolver(long long N_, long long F_, const int64_t *a, const
         // the persistent solve: one block per SM, all resident
         int coop = 0, occ = 0;
         GCK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev_id));
-        GCK(mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kg_solve_persistent<float>, kGpThreads, 0)
-                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kg_solve_persistent<double>, kGpThreads, 0));
+        GCK(cudaFuncSetAttribute(kg_solve_persistent<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGpRowBytes));
+        GCK(cudaFuncSetAttribute(kg_solve_persistent<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGpRowBytes));
+        GCK(mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kg_solve_persistent<float>, kGpThreads, kGpRowBytes)
+                  : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kg_solve_persistent<double>, kGpThreads, kGpRowBytes));
         if (coop && occ >= 1 && (int)lv.size() <= kGpLevels) {
             persist_blocks = sms;
             d_bar = dev<unsigned>(kGridBarWords + 1);  // the barrier's words, then the expired-wait word
@@ -1412,6 +1414,7 @@ void GeneralSolver::solve_persistent(const double *b, double *x, double tol2) {
     P.tol2 = tol2;
     P.maxiter = opt.maxiter;
     P.max_rounds = opt.max_outer;
+    P.row_bytes = kGpRowBytes;
     P.dir = lv[0].dir;
     P.b64 = b;
     P.x64 = x;
@@ -1434,6 +1437,7 @@ void GeneralSolver::solve_persistent(const double *b, double *x, double tol2) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(persist_blocks);
     cfg.blockDim = dim3(kGpThreads);
+    cfg.dynamicSmemBytes = kGpRowBytes;
     cfg.stream = stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;

@@ -92,3 +92,25 @@ def test_face_lists(gpu_lib, orc, kind, degree, precision):
     assert rel(got[0], want[0]) < 1e-8
     for g, w in zip(got[1:], want[1:]):
         assert rel(g, w) < 1e-6
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("degree", [1, 2, 3])
+def test_face_lists_levels_of_both_kinds(gpu_lib, degree, precision):
+    """90k cells: the finest level has more rows than half the threads of the GPU, the next ones fewer, the last ones
+    run in one block. Against the separate launches; both stop at 1e-12 of the right-hand side."""
+    i = np.arange(300 * 300).reshape(300, 300)
+    nb = np.concatenate([np.stack([i[:-1].ravel(), i[1:].ravel()], 1), np.stack([i[:, :-1].ravel(), i[:, 1:].ravel()], 1)])
+    n, rng = i.size, np.random.default_rng(2)
+    aol, Ks = rng.uniform(0.5, 2.0, len(nb)), np.exp(-9.0 + rng.standard_normal(len(nb)))
+    dn = np.concatenate([i[0], i[-1]])
+    dh, Qs = np.zeros(n), np.zeros(n)
+    dh[i[0]] = 1.0
+    Qs[i[100, 100]] = 1e-4
+    out = []
+    for graphs in (1, 0):
+        P = gpu_lib.GroundwaterProblem(nb, aol, dn, N=n, general=True, precision=precision, reltol=1e-12, cheb_degree=degree,
+                                       use_graphs=graphs)
+        out.append((P.forward(Ks, dh, Qs),) + tuple(P.adjoint(np.ones(n))))
+    for got, want in zip(*out):
+        assert rel(got, want) < 1e-8
