@@ -1614,7 +1614,9 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
                                             : (const void *)k_solve_persistent<float, false>)
                               : (nprob == 1 ? (const void *)k_solve_persistent<double, true>
                                             : (const void *)k_solve_persistent<double, false>);
-        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kPersistThreads, 0));
+        // (k is set to take kPersistTailBytes with a single problem)
+        if (nprob == 1) CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistTailBytes));
+        CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kPersistThreads, nprob == 1 ? kPersistTailBytes : 0));
         if (coop && occ >= 1 && nlev_max <= kPersistLevels && nprob <= std::min(sms, kPersistProblems)) persist_blocks = sms;
     }
     // fused tail: from the first level (>= 1) at which a problem has at most tail_cells cells
@@ -1801,6 +1803,7 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
     if (persist_blocks) {
         std::vector<int2> pt(nprob);
         for (int p = 0; p < nprob; p++) pt[p] = make_int2(ptail[p], nlev[p] - 1);
+        ptail0 = ptail[0];
         d_ptail = dalloc<int2>(nprob, owned);
         d_ppart = dalloc<double2>(2 * (size_t)std::max(pall.n, lv[0].psmooth.n), owned);
         CK(cudaMemcpy(d_ptail, pt.data(), nprob * sizeof(int2), cudaMemcpyHostToDevice));
@@ -2785,6 +2788,11 @@ void StructBatch::solve_persistent(const double *b, double *x, double tol2) {
     P.maxiter = opt.maxiter;
     P.max_rounds = opt.max_outer;
     P.zero_guess = zero_guess ? 1 : 0;
+    P.tail_bytes = 0;
+    if (nprob == 1)  // what stage_tail can use
+        for (int l = std::max(ptail0, 1); l < nlev_max; l++)
+            P.tail_bytes += (int)std::min<long long>(lv[l].h_desc[0].n, 1 << 16) * (sizeof(T) == 8 ? 81 : 29) + 16;
+    P.tail_bytes = std::min(P.tail_bytes, kPersistTailBytes);
     P.b64 = b;
     P.x64 = x;
     P.r = (T *)cgv[0];
@@ -2804,6 +2812,7 @@ void StructBatch::solve_persistent(const double *b, double *x, double tol2) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(persist_blocks);
     cfg.blockDim = dim3(kPersistThreads);
+    cfg.dynamicSmemBytes = P.tail_bytes;
     cfg.stream = stream;
     cfg.attrs = at;
     cfg.numAttrs = 1;

@@ -161,6 +161,7 @@ public:
     void solve_persistent(const double *b, double *x, double tol2);
     void build_pieces(Pieces &P, const std::vector<LevelDesc> &desc, const std::vector<int> &take);
     Pieces pall;                     // finest cells of every problem
+    int ptail0 = 0;                  // the first problem's
     int2 *d_ptail = nullptr;         // per problem {first level of its one-block tail, coarsest level}
     double2 *d_ppart = nullptr;      // its reduction slots
     int persist_blocks = 0;          // blocks of the cooperative launch (0: not available)
