@@ -13,6 +13,7 @@
 #include <string>
 
 #include "dpf_struct.h"
+#include "dpf_means.cuh"
 
 namespace dpf {
 
@@ -29,22 +30,6 @@ constexpr int kSolveRows = 32;     // rows of a forward block
 constexpr int kStepBuf = kNB * kNB + kNB;  // Z_TT and the pivots, behind a front's L columns
 
 int blocks_of(int n, int b) { return (n + b - 1) / b; }
-
-// 1 / p for a positive p: the reciprocal of p's significand from a float division, then one
-// third-order Householder step r (1 + e + e^2), e = 1 - m r (|e| < 2^-22, so its error is below
-// 2^-66 before rounding). Three FP64 instructions in a chain that every column waits for; the
-// division the compiler emits has about ten, 70 clocks each from a single warp. Exponents outside
-// +-500 (and zero, infinity, NaN) take the division.
-__device__ __forceinline__ double recip(double p) {
-    const long long u = __double_as_longlong(p);
-    const int ex = (int)((u >> 52) & 0x7FF);
-    if (ex < 523 || ex > 1523) return 1.0 / p;
-    const double m = __longlong_as_double((u & 0xFFFFFFFFFFFFFll) | 0x3FF0000000000000ll);
-    const double r = (double)(1.0f / (float)m);
-    const double e = fma(-m, r, 1.0);
-    const double q = fma(r, fma(e, e, e), r);
-    return __longlong_as_double(__double_as_longlong(q) + ((long long)(1023 - ex) << 52));
-}
 
 // ------------------------------------------------------------------ small fronts: one block each
 // The whole front in shared memory (column-major, odd leading dimension): its panel with the

@@ -1,4 +1,4 @@
-// dpf_means.cuh -- FP64 exponentials and face means with few FP64 instructions (a B300 SM issues 1.6 FP64
+// dpf_means.cuh -- FP64 exponentials, reciprocals and face means with few FP64 instructions (a B300 SM issues 1.6 FP64
 // lanes a clock, against 128 FP32 and 64 integer ones, so every kernel that evaluates them is bound by them).
 #pragma once
 #include "dpf_internal.h"
@@ -137,6 +137,22 @@ __device__ __forceinline__ double div64(double num, double den) {
     const double r = fma(fma(-den, r0, 1.0), r0, r0);
     const double q = num * r;
     return fma(fma(-den, q, num), r, q);
+}
+
+// 1 / p for a positive p: the reciprocal of p's significand from a float division, then one
+// third-order Householder step r (1 + e + e^2), e = 1 - m r (|e| < 2^-22, so its error is below
+// 2^-66 before rounding). Three FP64 instructions in a chain that a column's or a pivot's threads wait for; the
+// division the compiler emits has about ten, 70 clocks each from a single warp. Exponents outside
+// +-500 (and zero, infinity, NaN) take the division.
+__device__ __forceinline__ double recip(double p) {
+    const long long u = __double_as_longlong(p);
+    const int ex = (int)((u >> 52) & 0x7FF);
+    if (ex < 523 || ex > 1523) return 1.0 / p;
+    const double m = __longlong_as_double((u & 0xFFFFFFFFFFFFFll) | 0x3FF0000000000000ll);
+    const double r = (double)(1.0f / (float)m);
+    const double e = fma(-m, r, 1.0);
+    const double q = fma(r, fma(e, e, e), r);
+    return __longlong_as_double(__double_as_longlong(q) + ((long long)(1023 - ex) << 52));
 }
 
 // Face conductances from the cell values kc:

@@ -168,63 +168,82 @@ __global__ void k_coarsen(const LevelDesc *__restrict__ fdesc, const LevelDesc *
 }
 
 // ------------------------------------------------------ coarsest level
-// Dense inverse of each listed problem's coarsest operator (n <= 64), one block
-// per problem, by in-place Gauss-Jordan elimination in shared memory (no pivoting:
-// the operator is symmetric positive definite, so every pivot is a positive Schur
-// complement). The coarsest solve is then one small matrix-vector product.
-// The inverse is stored row-major with stride kMaxCoarse.
-__global__ void k_coarse_factor(const LevelDesc *__restrict__ desc, const int *__restrict__ plist,
+// Dense inverse of each listed problem's coarsest operator (n <= 64), one block per problem, by
+// symmetric sweeps in shared memory (no pivoting: the operator is symmetric positive definite, so every
+// pivot is a positive Schur complement): for pivot k, A_ij -= A_ik A_jk / A_kk, A_ik /= A_kk,
+// A_kk = -1 / A_kk; after the last one A is minus the inverse. The coarsest solve is then one small
+// matrix-vector product. The inverse is stored row-major with stride kMaxCoarse.
+// One SM's FP64 rate and the pivots' chain bound it: only the lower triangle is kept, and a pivot
+// touches the rows before it and those within the operator's bandwidth behind it (n^3 / 6 updates of the
+// n^3 of an elimination on all entries); two block barriers per pivot, the next pivot's column being
+// copied by the threads that update it. n = 49: 106 -> 43 us.
+__global__ void __launch_bounds__(kBlock) k_coarse_factor(const LevelDesc *__restrict__ desc, const int *__restrict__ plist,
                                 const double *__restrict__ cx, const double *__restrict__ cy,
                                 const double *__restrict__ cz, const double *__restrict__ leak, double *Inv,
                                 int *status) {
     pdl_enter();
-    __shared__ double A[kMaxCoarse][kMaxCoarse + 1];
-    __shared__ double col[kMaxCoarse];
-    __shared__ int bad;
-    int p = plist[blockIdx.x];
-    LevelDesc L = desc[p];
-    int n = (int)L.n;
-    const int sy = L.nz, sx = L.ny * L.nz;
-    for (int k = threadIdx.x; k < kMaxCoarse * kMaxCoarse; k += blockDim.x) A[k / kMaxCoarse][k % kMaxCoarse] = 0.0;
-    if (threadIdx.x == 0) bad = 0;
+    constexpr int kTri = kMaxCoarse * (kMaxCoarse + 1) / 2;
+    __shared__ double A[kMaxCoarse][kMaxCoarse + 1];  // lower triangle
+    __shared__ double col[2][kMaxCoarse], low[kMaxCoarse];  // pivot columns, and the present one over its pivot
+    __shared__ uint16_t at[kTri];  // row and column of the lower triangle's entries, row by row
+    const int p = plist[blockIdx.x], t = threadIdx.x;
+    const LevelDesc L = desc[p];
+    const int n = (int)L.n;
+    const int sy = L.nz, sx = L.ny * L.nz, band = L.nx > 1 ? sx : L.ny > 1 ? sy : 1;
+    for (int k = t; k < kMaxCoarse * kMaxCoarse; k += kBlock) {
+        const int i = k / kMaxCoarse, j = k % kMaxCoarse;
+        A[i][j] = 0.0;
+        if (j <= i) at[i * (i + 1) / 2 + j] = (uint16_t)(i << 8 | j);
+    }
     __syncthreads();
-    for (int li = threadIdx.x; li < n; li += blockDim.x) {
+    for (int li = t; li < n; li += kBlock) {
         int q = li / L.nz, iz = li - q * L.nz, iy = q % L.ny, ix = q / L.ny;
         long long i = L.off + li;
         double d = leak[i];
-        if (iz + 1 < L.nz) { double w = cz[i];      d += w; A[li][li + 1] = -w; }
+        if (iz + 1 < L.nz) d += cz[i];
         if (iz > 0)        { double w = cz[i - 1];  d += w; A[li][li - 1] = -w; }
-        if (iy + 1 < L.ny) { double w = cy[i];      d += w; A[li][li + sy] = -w; }
+        if (iy + 1 < L.ny) d += cy[i];
         if (iy > 0)        { double w = cy[i - sy]; d += w; A[li][li - sy] = -w; }
-        if (ix + 1 < L.nx) { double w = cx[i];      d += w; A[li][li + sx] = -w; }
+        if (ix + 1 < L.nx) d += cx[i];
         if (ix > 0)        { double w = cx[i - sx]; d += w; A[li][li - sx] = -w; }
         A[li][li] = d;
     }
     __syncthreads();
+    for (int i = t; i < n; i += kBlock) col[0][i] = A[i][0];
+    __syncthreads();
+    bool bad = false;
     for (int k = 0; k < n; k++) {
-        // pivot row k scaled by 1/A[k][k] (with the identity column folded in); save column k
-        double piv = A[k][k];
-        if (!(piv > 0.0)) { if (threadIdx.x == 0) bad = 1; piv = 1.0; }
-        double ip = 1.0 / piv;
-        __syncthreads();
-        for (int i = threadIdx.x; i < n; i += blockDim.x) col[i] = A[i][k];
-        __syncthreads();
-        for (int j = threadIdx.x; j < n; j += blockDim.x) A[k][j] = (j == k ? 1.0 : A[k][j]) * ip;
-        __syncthreads();
-        for (int t = threadIdx.x; t < n * n; t += blockDim.x) {
-            int i = t / n, j = t % n;
-            if (i == k) continue;
-            double rk = A[k][j];
-            A[i][j] = (j == k ? 0.0 : A[i][j]) - col[i] * rk;
+        const int m = min(n, k + band + 1);  // rows with an entry in column k
+        const double *c = col[k & 1];
+        double *next = col[~k & 1];
+        if (t < m) {
+            double piv = c[k];
+            if (!(piv > 0.0)) { bad = true; piv = 1.0; }
+            const double ip = recip(piv), v = t == k ? -ip : c[t] * ip;
+            low[t] = v;
+            if (t >= k) A[t][k] = v;
+            else A[k][t] = v;
         }
+        __syncthreads();
+        for (int e = t; e < m * (m + 1) / 2; e += kBlock) {
+            const int i = at[e] >> 8, j = at[e] & 255;
+            double v = A[i][j];
+            if (i != k && j != k) {
+                v = fma(-c[i], low[j], v);
+                A[i][j] = v;
+            }
+            if (j == k + 1) next[i] = v;
+            else if (i == k + 1) next[j] = v;
+        }
+        if (t == 0 && m < n) next[m] = A[m][k + 1];  // enters with the next pivot
         __syncthreads();
     }
     double *Ip = Inv + (long long)p * kMaxCoarse * kMaxCoarse;
-    for (int k = threadIdx.x; k < kMaxCoarse * kMaxCoarse; k += blockDim.x) {
-        int i = k / kMaxCoarse, j = k % kMaxCoarse;
-        Ip[k] = (i < n && j < n) ? A[i][j] : 0.0;
+    for (int k = t; k < kMaxCoarse * kMaxCoarse; k += kBlock) {
+        const int i = k / kMaxCoarse, j = k % kMaxCoarse;
+        Ip[k] = (i < n && j < n) ? -A[max(i, j)][min(i, j)] : 0.0;
     }
-    if (threadIdx.x == 0 && bad) atomicExch(status, 1);
+    if (bad) atomicExch(status, 1);
 }
 
 // ---- per-cell bodies of the V-cycle steps, shared by the per-level kernels (one launch

@@ -114,3 +114,19 @@ def test_face_lists_levels_of_both_kinds(gpu_lib, degree, precision):
         out.append((P.forward(Ks, dh, Qs),) + tuple(P.adjoint(np.ones(n))))
     for got, want in zip(*out):
         assert rel(got, want) < 1e-8
+
+
+@pytest.mark.parametrize("ns", [(1, 1, 2), (1, 1, 64), (1, 64, 1), (64, 1, 1), (7, 7, 1), (4, 4, 4), (2, 32, 1), (32, 1, 2), (3, 3, 7)])
+def test_coarsest_inverse(gpu_lib, orc, ns):
+    """Grids that are their own coarsest level: preconditioned with an exact inverse CG ends after one iteration, or two
+    should rounding (n eps cond, below 1e-10 here) leave more than the 1e-12 asked for."""
+    coords, nb, aol, _ = gpu_lib.regulargrid3d((0.0, 0.0, 0.0), (9.0, 8.0, 7.0), ns)
+    n, rng = coords.shape[1], np.random.default_rng(4)
+    Ks = np.exp(rng.standard_normal(len(nb)))
+    dh, Qs = np.zeros(n), rng.standard_normal(n)
+    dn = np.array([n // 2])
+    Qs[dn] = 0.0
+    P = gpu_lib.GroundwaterProblem.regular3d((0.0, 0.0, 0.0), (9.0, 8.0, 7.0), ns, dn, precision="fp64", reltol=1e-12)
+    h = P.forward(Ks, dh, Qs)
+    assert P.stats["iterations"] <= 2
+    assert rel(h, orc.Problem(n, nb, aol, dn).steady(Ks, dh, Qs, reltol=1e-14)) < 1e-9
