@@ -1,4 +1,4 @@
-// dpf_means.cuh -- FP64 exponentials, reciprocals and face means with few FP64 instructions (a B300 SM issues 1.6 FP64
+// dpf_means.cuh -- FP64 exponentials, powers, reciprocals and face means with few FP64 instructions (a B300 SM issues 1.6 FP64
 // lanes a clock, against 128 FP32 and 64 integer ones, so every kernel that evaluates them is bound by them).
 #pragma once
 #include "dpf_internal.h"
@@ -114,6 +114,123 @@ __device__ __forceinline__ double exp64(double x) {
     double p = fma(r, 1.0 / (24.0 * s * s * s * s), (1.0 / 6.0 + R * R / 96.0) / (s * s * s));
     p = fma(p, r, 1.0 / (2.0 * s * s));
     p = fma(p, r, (1.0 - R * R * R * R / 384.0) / s);
+    p *= r;
+    const int n = (int)nf;
+    const double2 t = kExp2Table[n & 255];
+    const double v = t.x + fma(t.x, p, t.y);
+    return __longlong_as_double(__double_as_longlong(v) + ((long long)(n >> 8) << 52));
+}
+
+// log x of a normal x as hi + lo with an absolute error near 2^-61, table-driven (P. T. P. Tang, ACM TOMS 16,
+// 1990): x = 2^k m, c_j about 1 / m to 9 bits, log x = k ln2 - log c_j + log1p(m c_j - 1); ln2 and the table
+// are split at 2^-42, so that the sum of their leading parts is exact. 16 FP64 instructions.
+struct LogDD {
+    double hi, lo;
+};
+static __device__ const double kLogTable[128][3] = {  // c, -log c rounded to a multiple of 2^-42, the rest
+    {0x1.0000000000000p+0, 0x0.0p+0, 0x0.0p+0}, {0x1.fa00000000000p-1, 0x1.82448a3880000p-7, 0x1.4554412c584e0p-44},
+    {0x1.f600000000000p-1, 0x1.432a925980000p-6, 0x1.98139928637fep-47}, {0x1.f200000000000p-1, 0x1.c63d2ec150000p-6, -0x1.5439ce030a687p-44},
+    {0x1.ef00000000000p-1, 0x1.149e3e4008000p-5, -0x1.2b98a9a4168fdp-44}, {0x1.eb00000000000p-1, 0x1.5715c4c040000p-5, -0x1.8888ddfc47628p-44},
+    {0x1.e700000000000p-1, 0x1.9a187b5740000p-5, -0x1.0c22e4ec4d90dp-44}, {0x1.e400000000000p-1, 0x1.ccb73cddd8000p-5, 0x1.965c36e09f5fep-44},
+    {0x1.e000000000000p-1, 0x1.08598b59e4000p-4, -0x1.7e5dd7009902cp-46}, {0x1.dd00000000000p-1, 0x1.2207b5c784000p-4, 0x1.49d8cfc10c7bfp-44},
+    {0x1.d900000000000p-1, 0x1.4485e03dbc000p-4, 0x1.fad46e8d26ab7p-44}, {0x1.d600000000000p-1, 0x1.5e95a4d978000p-4, 0x1.1cb7ce1d17171p-44},
+    {0x1.d200000000000p-1, 0x1.8197e2f410000p-4, -0x1.c0fe460d20041p-44}, {0x1.cf00000000000p-1, 0x1.9c0c32d4d4000p-4, -0x1.ab7c09e838668p-44},
+    {0x1.cc00000000000p-1, 0x1.b6ac88dad4000p-4, 0x1.b1bdff50225c7p-44}, {0x1.c900000000000p-1, 0x1.d179788218000p-4, 0x1.36433b5efbeedp-44},
+    {0x1.c600000000000p-1, 0x1.ec739830a0000p-4, 0x1.11fcba80cdd10p-44}, {0x1.c200000000000p-1, 0x1.08598b59e4000p-3, -0x1.7e5dd7009902cp-45},
+    {0x1.bf00000000000p-1, 0x1.160c8024b2000p-3, 0x1.ec2d2a9009e3dp-45}, {0x1.bc00000000000p-1, 0x1.23d712a49c000p-3, 0x1.00d238fd3df5cp-46},
+    {0x1.b900000000000p-1, 0x1.31b994d3a4000p-3, 0x1.f098ee3a50810p-44}, {0x1.b600000000000p-1, 0x1.3fb45a5992000p-3, 0x1.19713c0cae559p-44},
+    {0x1.b300000000000p-1, 0x1.4dc7b897bc000p-3, 0x1.c79b60ae1ff0fp-47}, {0x1.b100000000000p-1, 0x1.5737cc9018000p-3, 0x1.9baa7a6b887f6p-44},
+    {0x1.ae00000000000p-1, 0x1.6574ebe8c2000p-3, -0x1.98c1d34f0f462p-44}, {0x1.ab00000000000p-1, 0x1.73cb9074fe000p-3, -0x1.d66a90d0005a6p-44},
+    {0x1.a800000000000p-1, 0x1.823c16551a000p-3, 0x1.e0ddb9a631e83p-46}, {0x1.a500000000000p-1, 0x1.90c6db9fcc000p-3, -0x1.935f57718d7cap-46},
+    {0x1.a300000000000p-1, 0x1.9a8778deba000p-3, 0x1.470fa3efec390p-44}, {0x1.a000000000000p-1, 0x1.a93ed3c8ae000p-3, -0x1.8724350562169p-45},
+    {0x1.9d00000000000p-1, 0x1.b811730b82000p-3, 0x1.e90683b9cd768p-46}, {0x1.9b00000000000p-1, 0x1.c2028ab180000p-3, -0x1.92e0ee55c7ac6p-45},
+    {0x1.9800000000000p-1, 0x1.d1037f2656000p-3, -0x1.84a7e75b6f6e4p-47}, {0x1.9600000000000p-1, 0x1.db13db0d48000p-3, 0x1.2806a847527e6p-44},
+    {0x1.9300000000000p-1, 0x1.ea4449f04a000p-3, 0x1.5e91663732a36p-44}, {0x1.9100000000000p-1, 0x1.f474b134e0000p-3, -0x1.bae49f1df7b5ep-44},
+    {0x1.8e00000000000p-1, 0x1.01eae5626c000p-2, 0x1.a43dcfade85aep-44}, {0x1.8c00000000000p-1, 0x1.07138604d6000p-2, -0x1.e76324e912b17p-44},
+    {0x1.8a00000000000p-1, 0x1.0c42d67616000p-2, 0x1.7188b163ceae9p-45}, {0x1.8700000000000p-1, 0x1.14167ef367000p-2, 0x1.e0c07824daaf5p-44},
+    {0x1.8500000000000p-1, 0x1.1956d3b9bc000p-2, 0x1.7d2f73ad1aa14p-45}, {0x1.8300000000000p-1, 0x1.1e9e16788a000p-2, -0x1.82eaed3c8b65ep-44},
+    {0x1.8000000000000p-1, 0x1.269621134e000p-2, -0x1.1b61f10522625p-44}, {0x1.7e00000000000p-1, 0x1.2bef07cdc9000p-2, 0x1.a9cfa4a5004f4p-45},
+    {0x1.7c00000000000p-1, 0x1.314f1e1d36000p-2, -0x1.8e27ad3213cb8p-45}, {0x1.7a00000000000p-1, 0x1.36b6776be1000p-2, 0x1.16ecdb0f177c8p-46},
+    {0x1.7800000000000p-1, 0x1.3c25277333000p-2, 0x1.83b54b606bd5cp-46}, {0x1.7500000000000p-1, 0x1.44591e053a000p-2, -0x1.6e95892923d88p-47},
+    {0x1.7300000000000p-1, 0x1.49da7f3bcc000p-2, 0x1.07b334daf4b9ap-44}, {0x1.7100000000000p-1, 0x1.4f637ebbaa000p-2, -0x1.fc158cb3124b9p-44},
+    {0x1.6f00000000000p-1, 0x1.54f431b7be000p-2, 0x1.a8954c0910952p-46}, {0x1.6d00000000000p-1, 0x1.5a8cadbbee000p-2, -0x1.7c79b0af7ecf8p-48},
+    {0x1.6b00000000000p-1, 0x1.602d08af09000p-2, 0x1.ebe9176df3f65p-46}, {0x1.6900000000000p-1, 0x1.65d558d4ce000p-2, 0x1.544fd2dc5bdc0p-51},
+    {0x1.6700000000000p-1, 0x1.6b85b4cffa000p-2, 0x1.fe6750d372503p-45}, {0x1.6500000000000p-1, 0x1.713e33a46a000p-2, 0x1.7b9b2617e9472p-46},
+    {0x1.6300000000000p-1, 0x1.76feecb947000p-2, 0x1.74bb9c9852c57p-46}, {0x1.6100000000000p-1, 0x1.7cc7f7db47000p-2, -0x1.7c98438023cdcp-44},
+    {0x1.5f00000000000p-1, 0x1.82996d3ef9000p-2, -0x1.0d52aa30536bbp-44}, {0x1.5e00000000000p-1, 0x1.85855776dd000p-2, -0x1.015486666443bp-44},
+    {0x1.5c00000000000p-1, 0x1.8b639a88b3000p-2, -0x1.05ae1e5e70470p-45}, {0x1.5a00000000000p-1, 0x1.914a8635bf000p-2, 0x1.a2652b44673e1p-44},
+    {0x1.5800000000000p-1, 0x1.973a343135000p-2, 0x1.ab73b16bf4984p-44}, {0x1.5600000000000p-1, 0x1.9d32bea15f000p-2, -0x1.6279e10d0c0b0p-45},
+    {0x1.5400000000000p-1, 0x1.a334402250000p-2, -0x1.61cdd40314305p-44}, {0x1.5300000000000p-1, 0x1.a63865fabd000p-2, 0x1.d7bae3eeaa2e6p-47},
+    {0x1.5100000000000p-1, 0x1.ac478d0205000p-2, 0x1.bc0e8cc8a54afp-48}, {0x1.4f00000000000p-1, 0x1.b25fefb60d000p-2, -0x1.347cf9c45db45p-44},
+    {0x1.4e00000000000p-1, 0x1.b56fa04463000p-2, -0x1.bdab6b49ef99bp-44}, {0x1.4c00000000000p-1, 0x1.bb9611b80e000p-2, 0x1.7d85bf40a666dp-45},
+    {0x1.4a00000000000p-1, 0x1.c1c60693fa000p-2, 0x1.cec807fe8e180p-45}, {0x1.4900000000000p-1, 0x1.c4e19b8472000p-2, 0x1.e0d23293066a0p-45},
+    {0x1.4700000000000p-1, 0x1.cb200d2ceb000p-2, 0x1.90b9d9a2cb517p-44}, {0x1.4500000000000p-1, 0x1.d1684d49f4000p-2, 0x1.ab9d98a582718p-44},
+    {0x1.4400000000000p-1, 0x1.d490246df0000p-2, -0x1.652280b2c4c2cp-44}, {0x1.4200000000000p-1, 0x1.dae75484c9000p-2, 0x1.856f4a7c8e7a6p-44},
+    {0x1.4000000000000p-1, 0x1.e148a1a272000p-2, 0x1.b36537e3375b2p-44}, {0x1.3f00000000000p-1, 0x1.e47d1d32e6000p-2, 0x1.df865b95578b8p-44},
+    {0x1.3d00000000000p-1, 0x1.eaedd2eaca000p-2, -0x1.bcf314a1b2d37p-44}, {0x1.3c00000000000p-1, 0x1.ee2a156b41000p-2, 0x1.f27f45a470251p-45},
+    {0x1.3a00000000000p-1, 0x1.f4aa7ee032000p-2, -0x1.b4c86a43fad5dp-44}, {0x1.3900000000000p-1, 0x1.f7eeae6b57000p-2, 0x1.873001acabb96p-44},
+    {0x1.3700000000000p-1, 0x1.fe7f18eb04000p-2, -0x1.60f51ceb37e7ap-45}, {0x1.3600000000000p-1, 0x1.00e5ae5b20800p-1, -0x1.53ba3b1727b1cp-47},
+    {0x1.3400000000000p-1, 0x1.04360be760000p-1, 0x1.d6774030d58c4p-44}, {0x1.3300000000000p-1, 0x1.05e04c1aa3000p-1, -0x1.fcfe79d1ac1c7p-44},
+    {0x1.3200000000000p-1, 0x1.078bf0533c800p-1, -0x1.4bf6edf090501p-44}, {0x1.3000000000000p-1, 0x1.0ae76e2d05800p-1, -0x1.82de51de06076p-44},
+    {0x1.2f00000000000p-1, 0x1.0c974c8943000p-1, 0x1.cdc0a7cdcbb87p-45}, {0x1.2d00000000000p-1, 0x1.0ffb54213a800p-1, -0x1.c5108822a3283p-44},
+    {0x1.2c00000000000p-1, 0x1.11af823c75800p-1, 0x1.53cdc223111a7p-44}, {0x1.2b00000000000p-1, 0x1.1365252bf0800p-1, 0x1.930b4c43a97c2p-47},
+    {0x1.2900000000000p-1, 0x1.16d4d38c11800p-1, 0x1.fa75d42395d88p-45}, {0x1.2800000000000p-1, 0x1.188ee40f24000p-1, -0x1.accec41d52e6cp-44},
+    {0x1.2700000000000p-1, 0x1.1a4a738b7a000p-1, 0x1.9e2b126042793p-44}, {0x1.2500000000000p-1, 0x1.1dc619de06800p-1, 0x1.441b50bb38388p-45},
+    {0x1.2400000000000p-1, 0x1.1f8635fc61800p-1, -0x1.a7242c9fe81d3p-45}, {0x1.2300000000000p-1, 0x1.2147dba47a000p-1, 0x1.c9d579851b8b6p-44},
+    {0x1.2100000000000p-1, 0x1.24cfce6f81000p-1, -0x1.32cb5b2e5bdd7p-44}, {0x1.2000000000000p-1, 0x1.269621134d800p-1, 0x1.c93c1df5bb3b6p-44},
+    {0x1.1f00000000000p-1, 0x1.285e0842ca000p-1, 0x1.c1c4d866d5f22p-44}, {0x1.1e00000000000p-1, 0x1.2a2786d0ec000p-1, 0x1.06d2be797882dp-45},
+    {0x1.1c00000000000p-1, 0x1.2dbf557b0e000p-1, -0x1.7a6e507b9dc11p-46}, {0x1.1b00000000000p-1, 0x1.2f8dab6363000p-1, 0x1.bcccfdd1febc9p-44},
+    {0x1.1a00000000000p-1, 0x1.315da44340800p-1, -0x1.74e93c5a0ed9cp-45}, {0x1.1900000000000p-1, 0x1.332f4314ad800p-1, -0x1.a96c3d4e8a818p-47},
+    {0x1.1700000000000p-1, 0x1.36d77e9d35000p-1, -0x1.4a061506115f9p-48}, {0x1.1600000000000p-1, 0x1.38ae217197800p-1, -0x1.18b7abb5569a4p-45},
+    {0x1.1500000000000p-1, 0x1.3a86767257000p-1, 0x1.112e01e8919cap-45}, {0x1.1400000000000p-1, 0x1.3c6080c36c000p-1, -0x1.2b7367cfe13c2p-47},
+    {0x1.1300000000000p-1, 0x1.3e3c43918f800p-1, -0x1.27534c617cda4p-46}, {0x1.1200000000000p-1, 0x1.4019c2125c800p-1, 0x1.498c367879c5ap-44},
+    {0x1.1000000000000p-1, 0x1.43d9ff2f92000p-1, 0x1.e267b0b7efae1p-44}, {0x1.0f00000000000p-1, 0x1.45bcc464c8800p-1, 0x1.3a145b00234d8p-45},
+    {0x1.0e00000000000p-1, 0x1.47a1527e8a000p-1, 0x1.69a4a83594fabp-44}, {0x1.0d00000000000p-1, 0x1.4987ace0da800p-1, 0x1.d83ed15c6b2f4p-44},
+    {0x1.0c00000000000p-1, 0x1.4b6fd6f971000p-1, -0x1.f047750959d5fp-44}, {0x1.0b00000000000p-1, 0x1.4d59d43fda800p-1, 0x1.d0f65949c0a34p-44},
+    {0x1.0a00000000000p-1, 0x1.4f45a835a5000p-1, -0x1.e6c516d93b8fbp-45}, {0x1.0900000000000p-1, 0x1.5133566680000p-1, -0x1.d46359b33c2adp-44},
+    {0x1.0800000000000p-1, 0x1.5322e26867800p-1, 0x1.5ccc45d257531p-47}, {0x1.0700000000000p-1, 0x1.55144fdbcc000p-1, -0x1.4ec532b35ba3ep-44},
+    {0x1.0600000000000p-1, 0x1.5707a26bb9000p-1, -0x1.cccfe80199f84p-44}, {0x1.0500000000000p-1, 0x1.58fcddce00800p-1, -0x1.9e3900345a85dp-44},
+    {0x1.0400000000000p-1, 0x1.5af405c364800p-1, 0x1.dfa63ac10c9fbp-45}, {0x1.0300000000000p-1, 0x1.5ced1e17c3800p-1, -0x1.1d52fdabeaa73p-44},
+    {0x1.0200000000000p-1, 0x1.5ee82aa241800p-1, 0x1.202380cda46bep-45}, {0x1.0000000000000p-1, 0x1.62e42fefa3800p-1, 0x1.ef35793c76730p-45},
+};
+__device__ __forceinline__ LogDD log_dd(double x) {
+    const long long u = __double_as_longlong(x);
+    const double *t = kLogTable[(u >> 45) & 127];
+    const double m = __longlong_as_double((u & 0xFFFFFFFFFFFFFll) | 0x3FF0000000000000ll);
+    const double k = (double)((float)((int)(u >> 52) - 1023));
+    const double r = fma(m, t[0], -1.0);  // |r| <= 2^-7, rounded at 2^-61
+    const double h = fma(k, 0x1.62e42fefa3800p-1, t[1]);
+    const double s = h + r, e = r - (s - h);
+    double p = fma(r, -1.0 / 8.0, 1.0 / 7.0);
+    p = fma(p, r, -1.0 / 6.0);
+    p = fma(p, r, 1.0 / 5.0);
+    p = fma(p, r, -1.0 / 4.0);
+    p = fma(p, r, 1.0 / 3.0);
+    p = fma(p, r, -1.0 / 2.0);
+    p *= r * r;
+    return {s, e + (p + fma(k, 0x1.ef35793c76730p-45, t[2]))};
+}
+// x^y for x >= 0, and log x beside it, in 28 FP64 instructions against about 75 of the library's power; error 0.64 ulp
+// (0.56 for the logarithm). Zero, subnormal, infinite and NaN x and results beyond e^+-700 take the library's.
+__device__ __forceinline__ double pow64(double x, double y, LogDD &lx) {
+    const unsigned ex = (unsigned)(__double2hiint(x) >> 20);
+    if (ex - 23u > 2000u) {
+        lx = {log(x), 0.0};
+        return pow(x, y);
+    }
+    lx = log_dd(x);
+    const double z = y * lx.hi;
+    const float zf = (float)z;
+    if (!(fabsf(zf) < 700.0f)) return pow(x, y);
+    const double zl = fma(y, lx.lo, fma(y, lx.hi, -z));
+    constexpr double R = 0x1.63p-10;  // as in exp64
+    const float nf = rintf(zf * 369.32994f);
+    const double nd = (double)nf;
+    double r = fma(nd, -0x1.62e42fef80000p-9, z);
+    r = fma(nd, -0x1.1cf79abc9e3b4p-44, r) + zl;
+    double p = fma(r, 1.0 / 24.0, 1.0 / 6.0 + R * R / 96.0);
+    p = fma(p, r, 0.5);
+    p = fma(p, r, 1.0 - R * R * R * R / 384.0);
     p *= r;
     const int n = (int)nf;
     const double2 t = kExp2Table[n & 255];

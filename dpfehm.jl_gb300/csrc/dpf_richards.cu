@@ -40,21 +40,23 @@ struct Kr {
     double v, dpsi, dalpha, dN;
 };
 
-// FP64 arithmetic bounds the kernels that evaluate it (pow is ~100 FP64 instructions, and a B300 SM issues
-// 1.6 a clock): two powers per value, with u^N = u u^(N-1) and A^(-m/2) = sqrt(A^-m), and derivatives only
-// where they are used. With a power for each, and the derivatives always formed, the faces of a 200k-cell
-// grid (597k faces, two values each) took 895 us. u^(N-1) is the rounded one: N - 1 is exact for N >= 1/2,
-// and where u^N underflows u^(N-1) / u is still the right limit.
+// FP64 arithmetic bounds the kernels that evaluate it (a B300 SM issues 1.6 FP64 lanes a clock): two powers per
+// value, with u^N = u u^(N-1) and A^(-m/2) = sqrt(A^-m), table-driven ones (pow64, 28 instructions instead of the
+// library's 75), logarithms left over from them, and derivatives only where they are used. The faces of a
+// 200k-cell grid (597k faces, two values each) took 895 us with four library powers and all derivatives, 448 us
+// with two, 191 us now. u^(N-1) is the rounded one: N - 1 is exact for N >= 1/2, and where u^N underflows
+// u^(N-1) / u is still the right limit.
 template <KrWant kWant>
 __device__ Kr kr_vg(double psi, double alpha, double N) {
     Kr k{1.0, 0.0, 0.0, 0.0};
     if (!(psi < 0.0)) return k;
     const double m = (N - 1.0) / N;
     const double ap = fabs(alpha * psi);                 // u
-    const double uN1 = pow(ap, N - 1.0);
+    LogDD lu, lA;
+    const double uN1 = pow64(ap, N - 1.0, lu);
     const double uN = ap > 0.0 ? uN1 * ap : pow(ap, N);
     const double A = 1.0 + uN;
-    const double Am = pow(A, -m);
+    const double Am = pow64(A, -m, lA);
     const double numer = 1.0 - uN1 * Am;
     const double Amh = sqrt(Am);
     k.v = numer * numer * Amh;
@@ -69,11 +71,11 @@ __device__ Kr kr_vg(double psi, double alpha, double N) {
     k.dalpha = dkr_du * fabs(psi);
     // by N (m = 1 - 1/N, dm/dN = 1/N^2); u^N and u^(N-1) gain a factor ln u
     if (ap > 0.0) {
-        const double lu = log(ap), lA = log(A), dm = 1.0 / (N * N);
-        const double dA = uN * lu;
-        const double dAm = Am * (-dm * lA - m * dA * rA);
-        const double dnum = -(uN1 * lu * Am + uN1 * dAm);
-        const double dAmh = Amh * (-0.5 * dm * lA - 0.5 * m * dA * rA);
+        const double l = lu.hi + lu.lo, la = lA.hi + lA.lo, dm = 1.0 / (N * N);
+        const double dA = uN * l;
+        const double dAm = Am * (-dm * la - m * dA * rA);
+        const double dnum = -(uN1 * l * Am + uN1 * dAm);
+        const double dAmh = Amh * (-0.5 * dm * la - 0.5 * m * dA * rA);
         k.dN = 2.0 * numer * dnum * Amh + numer * numer * dAmh;
     }
     return k;
@@ -81,7 +83,7 @@ __device__ Kr kr_vg(double psi, double alpha, double N) {
 
 // Per face: Picard conductance K hm (kr_a, kr_b) and, with kJac, the flux-derivative parts of the Jacobian
 // (na, nb) and the face difference of the total head. FP64 arithmetic bounds it (see kr_vg): 597k faces
-// 448 us without the Jacobian and 527 us with it (895 us with the six powers and all derivatives).
+// 191 us without the Jacobian and 285 us with it.
 template <bool kJac>
 __global__ void kr_faces(int F, const int *__restrict__ fa, const int *__restrict__ fb,
                          const double *__restrict__ aol, const double *__restrict__ Ks,
@@ -248,7 +250,7 @@ __global__ void richards_mu_step(int n, const double *__restrict__ mnew, double 
 }
 
 // Face gradients with mu = -lambda (0 at Dirichlet cells): dK_f = H aol D (mu_a - mu_b);
-// dalpha_f, dN_f = K aol D (mu_a - mu_b) dH/d(.); bound by kr_vg's arithmetic (597k faces: 1000 -> 643 us)
+// dalpha_f, dN_f = K aol D (mu_a - mu_b) dH/d(.); bound by kr_vg's arithmetic (597k faces: 1000 -> 310 us)
 __global__ void richards_face_grads(int F, const int *__restrict__ fa, const int *__restrict__ fb,
                                     const double *__restrict__ aol, const double *__restrict__ Ks,
                                     const double *__restrict__ alphas, const double *__restrict__ Ns,

@@ -114,3 +114,21 @@ def test_van_genuchten_range(gpu_lib, nvg, psi_top, zero_alpha, solver):
     g = P.richards_adjoint(w, tol=1e-12)
     for got, want, name in zip(g, g_or, ("dKs", "ddirichletpsis", "dalphas", "dNs", "dQs")):
         assert rel(got, want) < 1e-7, name
+
+
+@pytest.mark.parametrize("N", [1.05, 1.5, 4.0, 9.0])
+def test_powers_of_the_whole_range(gpu_lib, N):
+    """One face between a free cell with a source and a Dirichlet cell at suction s, from 1e-100 (the powers of u are far
+    below the normal range) to 1e4, K scaled so that all fluxes are of order one: the oracle's flux at the returned psi
+    is the source. kr loses m u^-N to cancellation at large u, at most 1e-8 here: 4 eps / 1e-8 < 1e-6."""
+    for s in (1e-100, 1e-20, 1e-3, 1.0, 50.0, 1e4):
+        if (1 - 1 / N) * max(s, 1.0) ** -N < 1e-8:
+            continue
+        kd = ro.kr(np.array([-s]), 1.0, N)[0][0]
+        K, q = 1.0 / (kd * s), 1e-4
+        P = gpu_lib.GroundwaterProblem(np.array([[0, 1]]), np.ones(1), np.array([1]), N=2, general=True, reltol=1e-13)
+        psi = P.richards_steady(np.array([-s, -s]), np.array([K]), np.array([0.0, -s]), np.zeros(2), np.ones(1),
+                                np.array([N]), np.array([q, 0.0]), tol=1e-10, maxiter=50)
+        kf = ro.kr(psi[:1], 1.0, N)[0][0]
+        flux = K * 2 * kf * kd / (kf + kd) * (psi[0] + s)
+        assert abs(flux / q - 1.0) < 1e-6, (N, s)
