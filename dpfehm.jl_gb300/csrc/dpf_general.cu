@@ -10,7 +10,9 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
+#include <mutex>
 #include <numeric>
+#include <set>
 
 #include "dpf_direct.h"
 #include "dpf_front.h"
@@ -803,6 +805,20 @@ static void copy_out(double *dst, const double *src, size_t n, cudaStream_t s) {
         "copy out");
 }
 
+// function attributes, set once per device before any launch (never while another handle's kernels run or
+// are being captured)
+static void configure_persistent() {
+    static std::mutex mu;
+    static std::set<int> done;
+    int dev = 0;
+    GCK(cudaGetDevice(&dev));
+    std::lock_guard<std::mutex> lk(mu);
+    if (done.count(dev)) return;
+    for (const void *k : {(const void *)kg_solve_persistent<float>, (const void *)kg_solve_persistent<double>})
+        GCK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kGpRowBytes));
+    done.insert(dev);
+}
+
 GeneralSolver::GeneralSolver(long long N_, long long F_, const int64_t *a, const int64_t *b, const double *aol,
                              const double *volumes, long long nd, const int64_t *dn, const dpf_options &o,
                              cudaStream_t s)
@@ -851,8 +867,7 @@ GeneralSolver::GeneralSolver(long long N_, long long F_, const int64_t *a, const
         // the persistent solve: one block per SM, all resident
         int coop = 0, occ = 0;
         GCK(cudaDeviceGetAttribute(&coop, cudaDevAttrCooperativeLaunch, dev_id));
-        GCK(cudaFuncSetAttribute(kg_solve_persistent<float>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGpRowBytes));
-        GCK(cudaFuncSetAttribute(kg_solve_persistent<double>, cudaFuncAttributeMaxDynamicSharedMemorySize, kGpRowBytes));
+        configure_persistent();
         GCK(mixed ? cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kg_solve_persistent<float>, kGpThreads, kGpRowBytes)
                   : cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, kg_solve_persistent<double>, kGpThreads, kGpRowBytes));
         if (coop && occ >= 1 && (int)lv.size() <= kGpLevels) {

@@ -1633,8 +1633,6 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
                                             : (const void *)k_solve_persistent<float, false>)
                               : (nprob == 1 ? (const void *)k_solve_persistent<double, true>
                                             : (const void *)k_solve_persistent<double, false>);
-        // (k is set to take kPersistTailBytes with a single problem)
-        if (nprob == 1) CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistTailBytes));
         CK(cudaOccupancyMaxActiveBlocksPerMultiprocessor(&occ, k, kPersistThreads, nprob == 1 ? kPersistTailBytes : 0));
         if (coop && occ >= 1 && nlev_max <= kPersistLevels && nprob <= std::min(sms, kPersistProblems)) persist_blocks = sms;
     }
@@ -2071,6 +2069,8 @@ static void configure_kernels() {
     raise_pm_cheb<PM_PROLONG | PM_FIRST | PM_NOD>(raise);
     raise_pm_cheb<PM_PROLONG | PM_FIRST | PM_NOD | PM_RZ>(raise);
     raise_pm_cheb<PM_NOD | PM_RZ>(raise);
+    for (const void *k : {(const void *)k_solve_persistent<float, true>, (const void *)k_solve_persistent<double, true>})
+        CK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, kPersistTailBytes));
     raise((const void *)k_pm_restrict<float, 1>);
     raise((const void *)k_pm_restrict<float, 2>);
     raise((const void *)k_pm_restrict<float, 3>);
