@@ -6,7 +6,7 @@
 // (a forward and adjoint of the network 72 -> 43 ms, Richards' Picard and adjoint solves 63 -> 32 ms).
 // The finest level's steps are near the memory's rate (9..17 us each: gathers through the column indices);
 // a step on a small level takes 3..4 us, of which a barrier is 1.3. Those steps are bound by trips to L2:
-// a block keeps its rows of the small levels in shared memory, 2 to 8 lanes share a row, and the ranges of
+// a block keeps its rows of the small levels in shared memory, 2 to 8 lanes (FP64: 4) share a row, and the ranges of
 // a block's rows are worked out once (they cost two integer divisions per step). Together 51.3 -> 45.6 ms
 // and 34.3 -> 31.0 ms.
 //
@@ -154,10 +154,12 @@ struct GpSolve {
     __device__ __forceinline__ static bool small(int n, bool one) {
         return one || 64 * (((n + 31) / 32 + (int)gridDim.x - 1) / (int)gridDim.x) <= kGpThreads;
     }
-    // log2 of the lanes to a row where a block has m
+    // log2 of the lanes to a row where a block has m: at most 8, in FP64 at most 4 (the sums between the lanes are
+    // FP64 instructions too: 200k cells of Richards' equation 28.9 ms with 8, 28.1 with 4, 29.7 with 2, 35.4 with 1;
+    // a network of 815k mixed cells 45.1 ms with 4, 44.5 with 8, 44.4 with 16)
     __device__ __forceinline__ static int lanes(int m) {
         int lg = 0;
-        while (lg < 3 && (m << (lg + 1)) <= kGpThreads) lg++;
+        while (lg < (sizeof(T) == 8 ? 2 : 3) && (m << (lg + 1)) <= kGpThreads) lg++;
         return lg;
     }
     // Rows i0 .. i1 - 1. kSmall: 2 to 8 lanes to a row, f(row, lane, whether this thread stores the row's
