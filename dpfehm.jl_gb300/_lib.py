@@ -107,6 +107,7 @@ SIGNATURES = {
     "dpf_debug_expired_wait": (ctypes.c_int, [_f64p]),
     "dpf_debug_split48": (ctypes.c_int, [ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                          ctypes.c_void_p, ctypes.c_void_p]),
+    "dpf_debug_pow64": (ctypes.c_int, [ctypes.c_int64, _vp, _vp, _vp, _vp, _vp]),
     "dpf_debug_band_order_graph": (ctypes.c_int, [ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                                   ctypes.c_void_p]),
     "dpf_debug_band_order_grids": (ctypes.c_int, [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),

@@ -1,6 +1,6 @@
 // dpf_debug.cu -- test hooks: the bounded waits of the staging kernels, the integer-only
-// 48-bit split of doubles that the assembly and the round start use, and the band orderings of
-// the direct solver (host code, callable without a GPU).
+// 48-bit split of doubles that the assembly and the round start use, the table-driven power and
+// logarithm, and the band orderings of the direct solver (host code, callable without a GPU).
 //
 // dpf_debug_expired_wait runs one block whose threads wait on a shared-memory mbarrier
 // that nothing arrives on, through the same bounded wait (mbar_wait) that every staging
@@ -12,6 +12,7 @@
 #include <string>
 
 #include "dpf_direct.h"
+#include "dpf_means.cuh"
 #include "dpf_plane.cuh"
 
 namespace dpf {
@@ -42,7 +43,30 @@ __global__ void k_split48(long long n, const double *v, float *hi, float *lo, do
     v48[i] = w;
 }
 
+__global__ void k_pow64(long long n, const double *x, const double *y, double *p, double *lhi, double *llo) {
+    const long long i = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (i >= n) return;
+    LogDD l;
+    p[i] = pow64(x[i], y[i], l);
+    lhi[i] = l.hi;
+    llo[i] = l.lo;
+}
+
 }  // namespace dpf
+
+extern "C" int dpf_debug_pow64(int64_t n, const double *x, const double *y, double *p, double *log_hi, double *log_lo) {
+    if (n < 0 || (n > 0 && (!x || !y || !p || !log_hi || !log_lo))) return DPF_BAD_INPUT;
+    if (n == 0) return DPF_OK;
+    dpf::k_pow64<<<(unsigned)((n + 255) / 256), 256>>>((long long)n, x, y, p, log_hi, log_lo);
+    cudaError_t e = cudaGetLastError();
+    if (e == cudaSuccess) e = cudaDeviceSynchronize();
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        dpf::set_global_error(std::string("power probe: ") + cudaGetErrorString(e));
+        return DPF_CUDA;
+    }
+    return DPF_OK;
+}
 
 extern "C" int dpf_debug_split48(int64_t n, const double *v, float *hi, float *lo, double *v48, int *ok) {
     if (n < 0 || (n > 0 && (!v || !hi || !lo || !v48 || !ok))) return DPF_BAD_INPUT;

@@ -210,8 +210,10 @@ __device__ __forceinline__ LogDD log_dd(double x) {
     p *= r * r;
     return {s, e + (p + fma(k, 0x1.ef35793c76730p-45, t[2]))};
 }
-// x^y for x >= 0, and log x beside it, in 28 FP64 instructions against about 75 of the library's power; error 0.64 ulp
-// (0.56 for the logarithm). Zero, subnormal, infinite and NaN x and results beyond e^+-700 take the library's.
+// x^y for x >= 0, and log x beside it, in 28 FP64 instructions against about 75 of the library's power; error
+// 0.61 ulp (0.56 for the logarithm). |y| above 6 takes the library's: y lo, up to |y| 2^-15, takes r beyond the range R
+// that p is made for (0.66 ulp at |y| = 8, 1.0 at 16, 97 at 100, 2e6 at 1000; the library's is within 2), and so do
+// zero, subnormal, infinite and NaN x and results beyond e^+-700.
 __device__ __forceinline__ double pow64(double x, double y, LogDD &lx) {
     const unsigned ex = (unsigned)(__double2hiint(x) >> 20);
     if (ex - 23u > 2000u) {
@@ -219,6 +221,7 @@ __device__ __forceinline__ double pow64(double x, double y, LogDD &lx) {
         return pow(x, y);
     }
     lx = log_dd(x);
+    if ((__double2hiint(y) & 0x7FFFFFFF) > 0x40180000) return pow(x, y);  // 6.0, to 2^-18
     const double z = y * lx.hi;
     const float zf = (float)z;
     if (!(fabsf(zf) < 700.0f)) return pow(x, y);

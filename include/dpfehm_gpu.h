@@ -375,6 +375,11 @@ int dpf_debug_expired_wait(double *waited_ms);
  * (outputs then unspecified). All outputs are device arrays of n entries. */
 int dpf_debug_split48(int64_t n, const double *v, float *hi, float *lo, double *v48, int *ok);
 
+/* No counterpart in the reference. For n doubles x >= 0 and y (device memory) the power p = x^y of the
+ * relative-permeability kernels and the logarithm of x beside it, unevaluated (log_hi + log_lo). All
+ * outputs are device arrays of n entries. */
+int dpf_debug_pow64(int64_t n, const double *x, const double *y, double *p, double *log_hi, double *log_lo);
+
 /* No counterpart in the reference. The band orderings that size the direct solver, run on the host (no
  * device needed): for a symmetric graph in CSR form (rp[n + 1], ci, host arrays) the reverse
  * Cuthill-McKee order; for nprob regular grids (dims[3 p .. 3 p + 2] = nx, ny, nz, cells z fastest,
