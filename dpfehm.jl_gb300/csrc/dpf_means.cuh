@@ -287,16 +287,26 @@ __device__ __forceinline__ double face_mean_k(double ka, double kb, int kind) {
     return lo * (2.0 * div64(hi, ka + kb));
 }
 
-// dK_f / dlogK_a = dlogk_scale(ka) dlogk_weight(ka, kb): geometric K_f / 2 = (ka / 2) kb, harmonic
-// K_f^2 / (2 K_a) = 2 (ka t) t with t = kb / (ka + kb), in this order since t^2 could underflow; the scale is
-// applied once per cell, to the sum over its faces
+// dK_f / dlogK_a = dlogk_scale(ka) dlogk_weight(ka, kb), the scale applied once per cell, to the sum over its faces.
+//   geometric  K_f / 2: the weight is kb times ka's power of two, the scale half its significand, so that the weight is
+//              within a factor of two of K_f: kb alone times dK_f overflows or vanishes for cells hundreds of e-folds
+//              apart. Integer additions to the exponent; the FP64 instructions are those of kb alone.
+//   harmonic   K_f^2 / (2 ka) = 2 (ka t) t with t = kb / (ka + kb), in this order since t^2 could underflow
+__device__ __forceinline__ bool normal_exponent(int e) { return (unsigned)(e - 1) < 2046u; }
 __device__ __forceinline__ double dlogk_weight(double ka, double kb, int kind) {
-    if (kind == DPF_MEAN_GEOMETRIC) return kb;
+    if (kind == DPF_MEAN_GEOMETRIC) {
+        const int ea = __double2hiint(ka) >> 20, eb = __double2hiint(kb) >> 20;
+        if (normal_exponent(ea) && normal_exponent(eb) && normal_exponent(ea + eb - 1023))
+            return __longlong_as_double(__double_as_longlong(kb) + ((long long)(ea - 1023) << 52));
+        return (normal_exponent(ea) ? __longlong_as_double((long long)ea << 52) : ka) * kb;
+    }
     const double t = div64(kb, ka + kb);
     return ka * t * t;
 }
 __device__ __forceinline__ double dlogk_scale(double ka, int kind) {
-    return kind == DPF_MEAN_GEOMETRIC ? 0.5 * ka : 2.0;
+    if (kind != DPF_MEAN_GEOMETRIC) return 2.0;
+    const long long u = __double_as_longlong(ka);
+    return normal_exponent((int)(u >> 52)) ? __longlong_as_double((u & 0xFFFFFFFFFFFFFll) | 0x3FE0000000000000ll) : 0.5;
 }
 
 }  // namespace dpf

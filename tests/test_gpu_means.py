@@ -93,3 +93,31 @@ def test_arrays_in_place(gpu_lib, where):
            ctypes.c_void_p(raw.data_ptr() + g))
         got_g = get(g, n)
     assert np.array_equal(got_K, want_K) and np.array_equal(got_g, want_g)
+
+
+@pytest.mark.parametrize("general", [False, True])
+def test_pullback_of_cells_far_apart(gpu_lib, general):
+    """Geometric means of cells up to 1300 e-folds apart: K is moderate, but either cell's value times dK overflows or
+    vanishes. Also with a cell value that is 0 or subnormal, and a K that is. Twelve roundings as above."""
+    # in an order in which no two neighbouring rows of the grid have an infinite K
+    v = np.array([[-1200.0, 1199.0, 1e100], [1200.0, -1199.0, 1e-100], [-1300.0, 1299.0, -3e200], [1300.0, -1310.0, 2e-200],
+                  [-1400.0, 1380.0, 1e300], [-700.0, -720.0, 1e200], [-1500.0, 1400.0, 1e10], [0.3, 0.4, 1e-300],
+                  [-1430.0, 1400.0, 1e5]])
+    m = len(v)
+    logK = np.concatenate([v[:, 0], v[:, 1]])
+    if general:
+        nb, aol = np.stack([np.arange(m), np.arange(m) + m], 1), np.ones(m)
+        faces = np.arange(m)
+    else:
+        _, nb, aol, _ = gpu_lib.regulargrid3d((0.0, 0.0, 0.0), (1.0, 1.0, 1.0), (2, m, 1))
+        faces = np.nonzero(nb[:, 1] - nb[:, 0] == m)[0]
+    dKs = np.zeros(len(nb))
+    dKs[faces] = v[:, 2]
+    P = gpu_lib.GroundwaterProblem(nb, aol, np.array([0]), N=2 * m, general=general)
+    g = P.logk_to_faces_vjp(logK, dKs, "geometric")
+    k = np.exp(v[:, :2] / 2)                          # as the cells' values, 0 and subnormal ones among them
+    with np.errstate(all="ignore"):
+        want = 0.5 * k[:, 0].astype(np.longdouble) * k[:, 1] * v[:, 2]
+        sub = 2.0 ** -1074 * np.where(k < 1e-300, 1.0, 0.0).max(1) / np.maximum(k.min(1), 1e-323)  # rounding of exp itself
+    for got in (g[:m], g[m:]):
+        assert np.all(np.abs(got - want) <= (12 * EPS + 2 * sub) * np.abs(want) + 1e-300)
