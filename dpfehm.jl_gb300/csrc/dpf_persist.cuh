@@ -11,7 +11,8 @@
 //
 // Measured, forward + pullback, separate kernels -> one launch: FP64 50x50x5 3.42 -> 1.80 ms, 100x100x10
 // 4.57 -> 2.41 ms, 200x200x25 13.4 -> 7.2 ms, 20 grids of about 8k cells 4.41 -> 2.90 ms; mixed, 5
-// transient steps of 800k cells 46.6 -> 35.9 ms, 100x100x10 2.55 -> 2.03 ms.
+// transient steps of 800k cells 46.6 -> 35.9 ms, 100x100x10 2.55 -> 2.03 ms; 152 grids of 1000 cells FP64 2.97 -> 2.26 ms,
+// mixed 2.04 -> 1.70 ms.
 //
 // Per cell the arithmetic is that of the per-level kernels (the shared cell_* functions), so both
 // give the same iterates up to the order of the reductions; FP64 V-cycles of two steps take r D^-1 from
@@ -33,6 +34,7 @@ constexpr int kPersistTail32 = 2048, kPersistTail64 = 512;  // cells of a one-bl
 constexpr int kPersistTailBytes = 80 * 1024;  // shared memory for a single problem's tail
 constexpr int kPersistLevels = 16;
 constexpr int kPersistProblems = 256;  // (and at most one per block)
+static_assert(2 * kPersistProblems <= kPersistThreads, "two lanes per problem sum the slots");
 
 struct PersistSegs {
     const int4 *list;    // {problem, piece, pieces of the problem, 0}
@@ -63,7 +65,7 @@ struct PersistParams {
     unsigned *bar;
     int *expired;
     double2 *partials;   // two halves of nslots
-    int nslots;
+    int nslots, lane_bits;  // 1 << lane_bits lanes per problem sum its slots
     double tol2;
     int maxiter, max_rounds, zero_guess, tail_bytes;
     const double *b64;
@@ -264,24 +266,26 @@ struct Persist {
     }
     // The barrier behind a phase of sums: f(problem, state, total). One problem: every block adds the slots
     // up itself, in the same order, and keeps the problem's state in shared memory (2.8 us less than
-    // waiting for one block to do it); several: a warp per problem in the last block to arrive.
+    // waiting for one block to do it); several: 2 to 32 lanes per problem in the last block to arrive, so that all
+    // problems are summed at once (a warp per problem took 3.7 us for every 24 problems, four times an iteration).
     template <typename F>
     __device__ __forceinline__ bool reduce(const PersistSegs &S, F f, bool any = true) {
         if (!any) return bar.sync();
-        if (!single) return bar.sync([&] { totals(S, 0, kPersistThreads / 32, f); });
+        if (!single) return bar.sync([&] { totals(S, f); });
         if (!bar.sync()) return false;
-        if (threadIdx.x < 32) totals(S, 0, 1, f);
+        if (threadIdx.x < 32) total_of_one(S, f);
         // the next sums go to the other half: a slower block may still be reading this one
         half ^= 1;
         __syncthreads();
         return true;
     }
     __device__ __forceinline__ double2 *slots() const { return P.partials + (half ? P.nslots : 0); }
+    // one problem, by one warp (as a loop over problems: without it 1M FP64 cells took 0.8 % more, by its registers)
     template <typename F>
-    __device__ __forceinline__ void totals(const PersistSegs &S, int p0, int stride, F f) const {
+    __device__ __forceinline__ void total_of_one(const PersistSegs &S, F f) const {
         const int lane = threadIdx.x & 31;
 #pragma unroll 1
-        for (int p = p0 + (int)(threadIdx.x >> 5); p < P.nprob; p += stride) {
+        for (int p = (int)(threadIdx.x >> 5); p < P.nprob; p++) {
             const int2 g = single ? make_int2(0, S.n) : S.pinfo[p];
             if (g.y == 0) continue;
             double2 t = make_double2(0.0, 0.0);
@@ -295,6 +299,28 @@ struct Persist {
             t.y = warp_sum(t.y);
             if (lane == 0) f(p, st[p], t);
         }
+    }
+    // several problems, 1 << lane_bits lanes each
+    template <typename F>
+    __device__ __forceinline__ void totals(const PersistSegs &S, F f) const {
+        const int lg = P.lane_bits, p = (int)threadIdx.x >> lg, q = threadIdx.x & ((1 << lg) - 1);
+        // a warp without a problem has no sums to make (its FP64 additions would hold up the others')
+        if ((int)(threadIdx.x & ~31u) >> lg >= P.nprob) return;
+        const int2 g = p < P.nprob ? S.pinfo[p] : make_int2(0, 0);
+        double2 t = make_double2(0.0, 0.0);
+#pragma unroll 1
+        for (int k = q; k < g.y; k += 1 << lg) {
+            const double2 v = __ldcg(slots() + g.x + k);
+            t.x += v.x;
+            t.y += v.y;
+        }
+#pragma unroll
+        for (int l = 4; l >= 0; l--)
+            if (l < lg) {
+                t.x += __shfl_xor_sync(0xffffffffu, t.x, 1 << l);
+                t.y += __shfl_xor_sync(0xffffffffu, t.y, 1 << l);
+            }
+        if (q == 0 && g.y > 0) f(p, st[p], t);
     }
     template <typename V>
     __device__ __forceinline__ V scalar(const V *v) const {

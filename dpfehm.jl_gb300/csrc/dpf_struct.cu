@@ -2806,6 +2806,7 @@ void StructBatch::solve_persistent(const double *b, double *x, double tol2) {
     P.expired = d_factor_status + 1;
     P.partials = d_ppart;
     P.nslots = std::max(pall.n, lv[0].psmooth.n);
+    while (P.lane_bits < 5 && nprob << (P.lane_bits + 1) <= kPersistThreads) P.lane_bits++;
     P.tol2 = tol2;
     P.maxiter = opt.maxiter;
     P.max_rounds = opt.max_outer;

@@ -59,6 +59,16 @@ def test_batches(gpu_lib, orc, shapes, precision):
     _check(gpu_lib, orc, cases, precision=precision)
 
 
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("nprob", [24, 25, 48, 49, 96, 97, 152])
+def test_sums_of_many_problems(gpu_lib, orc, nprob, precision):
+    """Both sides of every change in the number of lanes that add up a problem's slots (32 down to 4). Problems of
+    different sizes and positions, so that a sum with another problem's slots would show."""
+    shapes = [((7, 5, 3), (6, 6, 4), (5, 4, 8))[k % 3] for k in range(nprob)]
+    cases = [steady_case(gpu_lib, ns, sigma=1.0, seed=k, ndir=1 + k % 2, nq=2) for k, ns in enumerate(shapes)]
+    _check(gpu_lib, orc, cases, precision=precision)
+
+
 def _mesh(kind):
     """(cells, faces, Dirichlet cells): a shuffled grid, a random tree, or pairs of cells beside a Dirichlet one
     (nothing to coarsen)."""
