@@ -457,7 +457,7 @@ int make_struct(const std::vector<GridSpec> &grids, const std::vector<std::vecto
                 Q->own_stream = true;
                 std::vector<GridSpec> g(grids.begin() + first, grids.begin() + first + cnt);
                 std::vector<std::vector<int64_t>> d(dn.begin() + first, dn.begin() + first + cnt);
-                Q->sb.reset(new StructBatch(g, d, Q->opt, Q->stream));
+                Q->sb.reset(new StructBatch(g, d, Q->opt, Q->stream, k));
                 P->part_first.push_back(first);
                 first += cnt;
             }

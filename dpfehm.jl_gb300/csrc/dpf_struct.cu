@@ -1577,6 +1577,7 @@ void StructBatch::build_pieces(Pieces &P, const std::vector<LevelDesc> &desc, co
     for (int p = 0; p < nprob; p++) {
         if (!take[p]) continue;
         const int k = (int)share[desc[p].n];
+        P.largest = std::max(P.largest, (desc[p].n + k - 1) / k);
         pinfo[p] = make_int2((int)list.size(), k);
         for (int q = 0; q < k; q++) list.push_back(make_int4(p, q, k, 0));
     }
@@ -1589,7 +1590,7 @@ void StructBatch::build_pieces(Pieces &P, const std::vector<LevelDesc> &desc, co
 }
 
 StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<std::vector<int64_t>> &dnodes,
-                         const dpf_options &o, cudaStream_t s)
+                         const dpf_options &o, cudaStream_t s, int parts)
     : opt(o), stream(s) {
     nprob = (int)grids.size();
     if (nprob <= 0) throw BadInput("empty batch");
@@ -1818,6 +1819,14 @@ StructBatch::StructBatch(const std::vector<GridSpec> &grids, const std::vector<s
     }
     // state, reductions, coarse factors
     d_state = dalloc<CgState>(nprob, owned);
+    if (persist_blocks) {
+        const int p = (int)(std::max_element(lv[0].h_desc.begin(), lv[0].h_desc.end(),
+                                             [](const LevelDesc &a, const LevelDesc &b) { return a.n < b.n; }) -
+                            lv[0].h_desc.begin());
+        const bool has_tail = tail_at[p] < nlev[p];
+        if (!persist_pays(parts, has_tail ? tail_at[p] : nlev[p] - 1, has_tail ? lv[tail_at[p]].h_desc[p].n : 0))
+            persist_blocks = 0;
+    }
     // active problems, -, loop passes, -; behind them the persistent kernel's barrier words
     d_count = dalloc<int>(kCountWords, owned);
     if (persist_blocks) {
@@ -2764,6 +2773,24 @@ void StructBatch::df_pcg(const double *b64, double *x64, double tol2) {
         }
         LAUNCH_CHECK();
     }
+}
+
+// Whether the one-launch solve of a batch is faster than the separate kernels, in microseconds per iteration. A step
+// of it lasts as long as its largest share (one share per block, at least one per problem: 77 problems on
+// 152 SMs take twice their even share), and concurrent parts run one after another, since each fills every SM; the
+// separate kernels spread any batch evenly and overlap, but pay for their launches (`levels` are smoothed by
+// launches of their own) and for a tail in one block per problem. Constants from 120 batches of 2 to 152 problems of
+// 60 to 1.5M cells, equal and uneven, as 1 to 3 parts, both forms measured: the form chosen is at most 8 % behind the other.
+// Without the rule, one launch -> separate: 150 problems of 1000 cells beside one of 1M FP64 323 -> 13.4 ms, mixed
+// 166 -> 8.0 ms; 77 of 40k cells FP64 31.3 -> 20.8 ms; 16 of 10k cells in 3 parts FP64 6.1 -> 3.7 ms; 4 of 1M mixed in 2
+// parts 18.5 -> 14.1 ms.
+bool StructBatch::persist_pays(int parts, int levels, long long tail_cells) const {
+    if (nprob == 1 && parts == 1) return true;
+    const double step = mixed ? 49.0 : 50.0;  // an iteration's barriers
+    const double share = 1e-3 * (mixed ? 6.0 : 16.0) * pall.largest;
+    const double even = 1e-3 * (mixed ? 1.5 : 18.0) * N / persist_blocks;
+    const double saved = mixed ? 36.0 + 3.0 * levels + 1.5e-3 * tail_cells : 8.0 * levels + 13e-3 * tail_cells;
+    return (parts - 1) * step + parts * (share - even) < std::max(saved, 5.0);
 }
 
 // ---- the whole solve in one launch (dpf_persist.cuh)

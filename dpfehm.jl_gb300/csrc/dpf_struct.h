@@ -76,6 +76,7 @@ public:
         int4 *list = nullptr;
         int2 *pinfo = nullptr;
         int n = 0;
+        long long largest = 0;  // cells of the largest share
     };
     struct Level {
         Pieces psmooth, prestr;  // cells of the smoothed problems; of their next level
@@ -101,8 +102,9 @@ public:
         void *work[4] = {nullptr, nullptr, nullptr, nullptr};   // xa, xb, b, d (V-cycle precision)
     };
 
+    // parts: the handles of a split batch that solve at the same time, this one among them
     StructBatch(const std::vector<GridSpec> &grids, const std::vector<std::vector<int64_t>> &dnodes,
-                const dpf_options &opt, cudaStream_t stream);
+                const dpf_options &opt, cudaStream_t stream, int parts = 1);
     ~StructBatch();
     StructBatch(const StructBatch &) = delete;
     StructBatch &operator=(const StructBatch &) = delete;
@@ -157,6 +159,7 @@ public:
     bool direct_tried = false, direct_stale = true, direct_ok = false;
     // one cooperative launch for the whole solve; use_persist: where it is the faster form
     bool use_persist() const;
+    bool persist_pays(int parts, int levels, long long tail_cells) const;
     template <typename T>
     void solve_persistent(const double *b, double *x, double tol2);
     void build_pieces(Pieces &P, const std::vector<LevelDesc> &desc, const std::vector<int> &take);

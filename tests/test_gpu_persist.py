@@ -69,6 +69,35 @@ def test_sums_of_many_problems(gpu_lib, orc, nprob, precision):
     _check(gpu_lib, orc, cases, precision=precision)
 
 
+@pytest.mark.parametrize("shapes,streams,precision,one_launch", [
+    ([(5, 5, 4)] * 150 + [(100, 100, 20)], 0, "fp64", False),     # one share would hold 13 even ones
+    ([(5, 5, 4)] * 150 + [(100, 100, 20)], 0, "mixed", False),
+    ([(30, 30, 10)] * 77, 0, "fp64", False),                      # twice the even share
+    ([(30, 30, 10)] * 77, 0, "mixed", False),
+    ([(30, 30, 10)] * 76, 0, "fp64", True),
+    ([(12, 10, 6)] * 4, 2, "fp64", False),                        # small parts: each would fill the GPU in turn
+    ([(12, 10, 6)] * 4, 2, "mixed", False),
+    ([(120, 120, 10)] * 4, 2, "fp64", True),                      # large ones: one-launch solves on two streams
+    ([(120, 120, 10)] * 4, 3, "fp64", False),
+])
+def test_form_of_a_batch(gpu_lib, shapes, streams, precision, one_launch):
+    """Batches whose shares or parts the one-launch solve would leave waiting take the separate kernels (some
+    hundred launches); either form, also from several host threads and streams, gives the host-driven loop's result.
+    Both solve to 1e-12; tolerances as above."""
+    cases = [steady_case(gpu_lib, ns, sigma=1.0, seed=k % 5, ndir=1 + k % 2, nq=2) for k, ns in enumerate(shapes)]
+    B, obs, h, g = _solve(gpu_lib, cases, precision=precision, streams=streams)
+    launches = B.launch_count
+    assert (launches < 60 * max(streams, 1)) == one_launch
+    B0, _, h0, g0 = _solve(gpu_lib, cases, use_graphs=0, precision=precision)
+    off = B.cell_offsets
+    cat = lambda k: np.concatenate([c[k] for c in cases])
+    for _ in range(3):
+        for k in range(len(cases)):
+            s = slice(off[k], off[k + 1])
+            assert rel(h[s], h0[s]) < 1e-10 and rel(g[s], g0[s]) < 1e-8, k
+        h, g = (np.asarray(v) for v in B.solve_grad_logk(cat("logK"), cat("dh"), cat("Qs"), obs))
+
+
 def _mesh(kind):
     """(cells, faces, Dirichlet cells): a shuffled grid, a random tree, or pairs of cells beside a Dirichlet one
     (nothing to coarsen)."""
