@@ -95,7 +95,7 @@ __device__ __forceinline__ void pass_first(const PersistParams<T> &P, const Pers
                 const T *u = V.d;
                 const T ui = u[c.i];
                 T dg;
-                const T t = resid7(L, c, V.C, T(0), ui, [&](long long j, int, int, int) { return u[j]; }, dg);
+                const T t = resid7(L, c, V.C, [] { return T(0); }, ui, [&](long long j, int, int, int) { return u[j]; }, dg);
                 const T r = fma(P.invtheta, t, b[c.i]);
                 V.xb[c.i] = fma(P.c2[1] * V.C.idg[c.i], r, P.u1 * ui);
                 continue;
@@ -188,7 +188,7 @@ __device__ __forceinline__ void pass_restrict(const PersistParams<T> &P, const P
                     if (c.iz < L.nz) {
                         c.i = L.off + ((long long)c.ix * L.ny + c.iy) * L.nz + c.iz;
                         T dg;
-                        const T r = resid7(L, c, V.C, b[c.i], cur[c.i],
+                        const T r = resid7(L, c, V.C, [&] { return b[c.i]; }, cur[c.i],
                                            [&](long long j, int, int, int) { return cur[j]; }, dg);
                         v = z ? v + r : r;
                     }

@@ -284,14 +284,14 @@ __device__ __forceinline__ void cell_cheb_first2(const LevelDesc &L, const Cell 
     T dg;
     if constexpr (sizeof(T) == 8) {
         const T u = bi * gi;  // x1 = invtheta u
-        const T t = resid7(L, c, C, T(0), u, [&](long long j, int, int, int) { return ldv<CG>(b, j) * g[j]; }, dg);
+        const T t = resid7(L, c, C, [] { return T(0); }, u, [&](long long j, int, int, int) { return ldv<CG>(b, j) * g[j]; }, dg);
         const T e = fma(c2, fma(invtheta, t, bi), c1 * invtheta * bi);
         d[c.i] = e;
         xout[c.i] = fma(gi, e, invtheta * u);
     } else {
         const T x1 = invtheta * bi * gi;
-        const T r = resid7(L, c, C, bi, x1, [&](long long j, int, int, int) { return invtheta * ldv<CG>(b, j) * g[j]; },
-                           dg);
+        const T r = resid7(L, c, C, [&] { return bi; }, x1,
+                           [&](long long j, int, int, int) { return invtheta * ldv<CG>(b, j) * g[j]; }, dg);
         const T dn = c1 * x1 + c2 * r * gi;
         d[c.i] = dn;
         xout[c.i] = x1 + dn;
@@ -304,8 +304,8 @@ __device__ __forceinline__ T cell_cheb_step(const LevelDesc &L, const Cell &c, c
                                             const T *__restrict__ b, const T *__restrict__ xin,
                                             T *__restrict__ xout, T *__restrict__ d, T c1, T c2, T &bi) {
     T xi = ldv<CG>(xin, c.i), dg;
-    bi = ldv<CG>(b, c.i);
-    const T ri = resid7(L, c, C, bi, xi, [&](long long j, int, int, int) { return ldv<CG>(xin, j); }, dg);
+    const T ri = resid7(L, c, C, [&] { return bi = ldv<CG>(b, c.i); }, xi,
+                        [&](long long j, int, int, int) { return ldv<CG>(xin, j); }, dg);
     T dn, xo;
     if constexpr (sizeof(T) == 8) {
         dn = FIRST ? c2 * ri : fma(c2, ri, c1 * ldv<CG>((const T *)d, c.i));
@@ -335,8 +335,8 @@ __device__ __forceinline__ T cell_restrict(const LevelDesc &L, const Cell &cc, c
                 c.ix = fx; c.iy = fy; c.iz = fz;
                 c.i = L.off + fx * fsx + fy * fsy + fz;
                 T xi = ldv<CG>(x, c.i), dg;
-                acc += resid7(L, c, C, ldv<CG>(b, c.i), xi, [&](long long j, int, int, int) { return ldv<CG>(x, j); },
-                              dg);
+                acc += resid7(L, c, C, [&] { return ldv<CG>(b, c.i); }, xi,
+                              [&](long long j, int, int, int) { return ldv<CG>(x, j); }, dg);
             }
     return acc;
 }

@@ -270,14 +270,16 @@ __device__ __forceinline__ void apply7(const LevelDesc &L, const Cell &c, const 
 // instructions against 14: GB300 issues 1.6 of them per clock and SM, which bounds every FP64 smoother. The
 // cancellation that the flux form avoids is in the last bits of diag_i x_i, and the V-cycle only
 // preconditions: CG's own products and residuals keep the flux form.
-template <typename T, typename XAt>
-__device__ __forceinline__ T resid7(const LevelDesc &L, const Cell &c, const Coeffs<T> &C, T bi, T xi, XAt xat,
+// bat() loads b_i: FP32 levels do so behind the product (held across it, it spilled in the per-level kernels, whose 32
+// registers are full: restriction of 1.2M cells 15.6 -> 17.3 us, first step behind the prolongation 11.8 -> 13.6 us).
+template <typename T, typename BAt, typename XAt>
+__device__ __forceinline__ T resid7(const LevelDesc &L, const Cell &c, const Coeffs<T> &C, BAt bat, T xi, XAt xat,
                                     T &diag) {
     if constexpr (sizeof(T) == 8) {
         const long long i = c.i;
         const long long sy = L.nz, sx = (long long)L.ny * L.nz;
         diag = T(0);
-        T r = fma(-C.dg[i], xi, bi);
+        T r = fma(-C.dg[i], xi, bat());
 #if DPF_CHECKED
         if (!(DPF_INSIDE(CK_NEIGHBOUR, c.iz + 1 < L.nz ? i + 1 : i, L.off, L.off + L.n) &&
               DPF_INSIDE(CK_NEIGHBOUR, c.iz > 0 ? i - 1 : i, L.off, L.off + L.n) &&
@@ -297,7 +299,7 @@ __device__ __forceinline__ T resid7(const LevelDesc &L, const Cell &c, const Coe
     } else {
         T Ax;
         apply7(L, c, C, xi, xat, Ax, diag);
-        return bi - Ax;
+        return bat() - Ax;
     }
 }
 
