@@ -105,6 +105,8 @@ SIGNATURES = {
     "dpf_debug_fail_alloc": (None, [ctypes.c_int64]),
     "dpf_debug_alloc_stats": (None, [ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]),
     "dpf_debug_expired_wait": (ctypes.c_int, [_f64p]),
+    "dpf_debug_expired_barrier": (ctypes.c_int, [ctypes.c_int, _f64p]),
+    "dpf_debug_expire_barriers": (ctypes.c_int, [_vp, ctypes.c_int]),
     "dpf_debug_split48": (ctypes.c_int, [ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                          ctypes.c_void_p, ctypes.c_void_p]),
     "dpf_debug_pow64": (ctypes.c_int, [ctypes.c_int64, _vp, _vp, _vp, _vp, _vp]),

@@ -212,6 +212,14 @@ extern "C" int dpf_debug_check_report(int64_t *violations, int64_t *first) {
 
 extern "C" void dpf_debug_fail_alloc(int64_t k) { dpf::g_fail_in.store(k < 0 ? -1 : (long long)k); }
 
+extern "C" int dpf_debug_expire_barriers(dpf_problem *P, int on) {
+    if (!P) return DPF_BAD_INPUT;
+    for (dpf_problem *Q : P->parts) dpf_debug_expire_barriers(Q, on);
+    if (P->sb) P->sb->barrier_short = on != 0;
+    if (P->gs) P->gs->barrier_short = on != 0;
+    return DPF_OK;
+}
+
 extern "C" void dpf_debug_alloc_stats(int64_t *made, int64_t *live) {
     if (made) *made = dpf::g_made.load();
     if (live) *live = dpf::g_live.load();

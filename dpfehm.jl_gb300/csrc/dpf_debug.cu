@@ -5,13 +5,15 @@
 // dpf_debug_expired_wait runs one block whose threads wait on a shared-memory mbarrier
 // that nothing arrives on, through the same bounded wait (mbar_wait) that every staging
 // kernel uses, so that a test sees that wait end by its bound, the error word set and the
-// device still usable, without any kernel of a solve being made to fail.
+// device still usable, without any kernel of a solve being made to fail. dpf_debug_expired_barrier
+// does the same for the grid barrier of the one-launch solves, with one block that never arrives.
 #include <cuda_runtime.h>
 
 #include <new>
 #include <string>
 
 #include "dpf_direct.h"
+#include "dpf_grid.cuh"
 #include "dpf_means.cuh"
 #include "dpf_plane.cuh"
 
@@ -30,6 +32,16 @@ __global__ void k_expired_wait(int *err, unsigned long long *waited_ns) {
         waited_ns[0] = global_ns() - t0;
         if (done) atomicExch(err, 2);  // the phase cannot complete: a defect of the wait
     }
+}
+
+// out: {error word, threads that saw the wait expire}, ns: the longest wait
+__global__ void k_expired_barrier(unsigned *words, int *out, unsigned long long *ns, int with_last) {
+    if (blockIdx.x == 0) return;  // never arrives
+    GridBar bar{words, out};
+    const uint64_t t0 = global_ns();
+    const bool got = with_last ? bar.sync([] {}) : bar.sync();
+    if (!got) atomicAdd(&out[1], 1);
+    if (threadIdx.x == 0) atomicMax(ns, (unsigned long long)(global_ns() - t0));
 }
 
 __global__ void k_split48(long long n, const double *v, float *hi, float *lo, double *v48, int *ok) {
@@ -118,6 +130,47 @@ extern "C" int dpf_debug_expired_wait(double *waited_ms) {
         return DPF_STATE;
     }
     dpf::set_global_error("a bounded staging wait expired after " + std::to_string(1e-6 * (double)h_ns) + " ms");
+    return DPF_TIMEOUT;
+}
+
+extern "C" int dpf_debug_expired_barrier(int with_last, double *waited_ms) {
+    int ndev = 0;
+    if (cudaGetDeviceCount(&ndev) != cudaSuccess || ndev == 0) {
+        cudaGetLastError();
+        dpf::set_global_error("no CUDA device");
+        return DPF_NO_DEVICE;
+    }
+    constexpr int kBlocks = 8, kThreads = 64;
+    constexpr size_t kBytes = dpf::kGridBarWords * sizeof(unsigned) + 16;
+    char *buf = nullptr;
+    if (dpf::dev_malloc((void **)&buf, kBytes) != cudaSuccess) {
+        cudaGetLastError();
+        dpf::set_global_error("device allocation failed");
+        return DPF_OOM;
+    }
+    unsigned *words = (unsigned *)buf;
+    unsigned long long *d_ns = (unsigned long long *)(buf + dpf::kGridBarWords * sizeof(unsigned));
+    int *d_out = (int *)(d_ns + 1);
+    int h_out[2] = {-1, -1};
+    unsigned long long h_ns = 0;
+    void *args[] = {&words, &d_out, &d_ns, &with_last};
+    cudaError_t e = cudaMemset(buf, 0, kBytes);
+    if (e == cudaSuccess)
+        e = cudaLaunchCooperativeKernel((const void *)dpf::k_expired_barrier, dim3(kBlocks), dim3(kThreads), args, 0, 0);
+    if (e == cudaSuccess) e = cudaMemcpy(h_out, d_out, sizeof(h_out), cudaMemcpyDeviceToHost);
+    if (e == cudaSuccess) e = cudaMemcpy(&h_ns, d_ns, sizeof(h_ns), cudaMemcpyDeviceToHost);
+    dpf::dev_free(buf);
+    if (e != cudaSuccess) {
+        cudaGetLastError();
+        dpf::set_global_error(std::string("expired-barrier probe: ") + cudaGetErrorString(e));
+        return DPF_CUDA;
+    }
+    if (waited_ms) *waited_ms = 1e-6 * (double)h_ns;
+    if (h_out[0] != 1 || h_out[1] != (kBlocks - 1) * kThreads) {
+        dpf::set_global_error("the grid barrier did not report its expiry to every thread");
+        return DPF_STATE;
+    }
+    dpf::set_global_error("a grid barrier expired after " + std::to_string(1e-6 * (double)h_ns) + " ms");
     return DPF_TIMEOUT;
 }
 

@@ -14,7 +14,9 @@ constexpr uint32_t kGridWaitTries = 1u << 28;    // ... or, should the global ti
 // Every thread of every block calls sync(last) the same number of times. The last block to arrive runs
 // last() (all its threads) before the others go on: the reductions of a phase are finished there, so
 // they need no barrier of their own. False (in every thread of the block) when the wait ran out: the
-// error word is set and the kernel returns; the other blocks' waits run out the same way.
+// error word is set and the kernel returns; the other blocks' waits run out the same way. The limit is wall time: it
+// also runs out where other work holds the SMs that the missing blocks wait for, or a phase of the solve itself
+// takes longer. The host then finishes the solve with the separate kernels, in which no block waits for another.
 struct GridBar {
     unsigned *words;
     int *err;

@@ -2856,6 +2856,7 @@ void StructBatch::solve_persistent(const double *b, double *x, double tol2) {
     P.cdf = CoeffsDF{cdf[0], cdf[1], cdf[2], cdf[3]};
     P.C64 = coeffs_of<double>(lv[0], true);
     CK(cudaMemsetAsync(d_count, 0, kCountWords * sizeof(int), stream));
+    if (barrier_short) CK(cudaMemsetAsync(P.bar, 0xff, sizeof(unsigned), stream));  // arrivals counted from -1
     cudaLaunchAttribute at[1];
     at[0].id = cudaLaunchAttributeCooperative;
     at[0].val.cooperative = 1;
@@ -2880,24 +2881,32 @@ void StructBatch::solve(const double *b, double *x, double reltol) {
         bool &f;
         ~ZeroGuessReset() { f = false; }
     } zg{zero_guess};
-    const bool persist = use_persist();
-    if (!persist) {
-        KTimer _kt(this, kname("k_state_init", 0, false), 0);
-        launch_pdl(k_state_init, (nprob + 127) / 128, 128, 0, stream, d_state, nprob);
-    }
-    LAUNCH_CHECK();
-    CK(cudaMemsetAsync(d_factor_status + 1, 0, sizeof(int), stream));  // expired-wait word of this solve
+    stats_outer = 0;
     graph_body_kernels = 0;
     stats_fresh = false;
-    if (persist) {
+    bool done = false;
+    CK(cudaMemsetAsync(d_factor_status + 1, 0, sizeof(int), stream));  // expired-wait word of this solve
+    if (use_persist()) {
         if (mixed) solve_persistent<float>(b, x, tol2);
         else solve_persistent<double>(b, x, tol2);
-        stats_outer = 0;
-    } else if (!mixed) {
-        pcg<double>(b, x, tol2);
-        stats_outer = 0;
-    } else {
-        df_pcg(b, x, tol2);
+        read_stats();
+        stats_fresh = done = !h_misc[1];
+        if (!done) {
+            // a barrier's limit ran out (dpf_grid.cuh): solved by the separate kernels from what x holds now, and
+            // so is every later solve of the handle, rather than after another second's wait
+            persist_blocks = 0;
+            zero_guess = false;
+            CK(cudaMemsetAsync(d_factor_status + 1, 0, sizeof(int), stream));
+        }
+    }
+    if (!done) {
+        {
+            KTimer _kt(this, kname("k_state_init", 0, false), 0);
+            launch_pdl(k_state_init, (nprob + 127) / 128, 128, 0, stream, d_state, nprob);
+        }
+        LAUNCH_CHECK();
+        if (mixed) df_pcg(b, x, tol2);
+        else pcg<double>(b, x, tol2);
     }
     // statistics, the error words and the graph passes in one synchronisation (already read when
     // the rounds ended on reading them)
@@ -2923,7 +2932,7 @@ void StructBatch::solve(const double *b, double *x, double reltol) {
     }
     if (h_misc[1]) {
         last_status = DPF_TIMEOUT;
-        last_message = "a bounded wait of a solver kernel (staging or grid barrier) expired";
+        last_message = "a shared-memory staging wait of a smoother kernel expired";
     }
 }
 

@@ -168,6 +168,7 @@ public:
     int2 *d_ptail = nullptr;         // per problem {first level of its one-block tail, coarsest level}
     double2 *d_ppart = nullptr;      // its reduction slots
     int persist_blocks = 0;          // blocks of the cooperative launch (0: not available)
+    bool barrier_short = false;      // test hook: one arrival too few
     cudaGraphExec_t loop_graph(int kind, void *x);
     void run_loop(int kind, void *x);
     int read_count(int which);

@@ -367,6 +367,17 @@ void dpf_debug_alloc_stats(int64_t *made, int64_t *live);
  * *waited_ms (may be NULL); any other status is a defect. The device stays usable. */
 int dpf_debug_expired_wait(double *waited_ms);
 
+/* No counterpart in the reference. The same for the barrier between the blocks of a one-launch solve (with_last: the
+ * form with work in the last block to arrive): eight blocks, one of which never arrives. DPF_TIMEOUT when every
+ * thread of the others saw the wait end (after one second), with the longest wait in *waited_ms (may be NULL);
+ * DPF_STATE for a defect. The device stays usable. */
+int dpf_debug_expired_barrier(int with_last, double *waited_ms);
+
+/* No counterpart in the reference. on != 0: the barriers of the handle's one-launch solves count one arrival too few, so
+ * that the next such solve gives up after one second. It is then finished by the separate kernels, as are the
+ * handle's later ones. */
+int dpf_debug_expire_barriers(dpf_problem *p, int on);
+
 /* No counterpart in the reference. For n doubles v (device memory) the split that the
  * mixed-precision assembly and round start use: v48 = v rounded to 48 significant bits
  * (to nearest, ties away from zero), hi + lo = v48 exactly (two floats), formed with integer

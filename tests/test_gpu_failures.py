@@ -150,3 +150,53 @@ def test_expired_wait_reports_timeout(gpu_lib, lib):
     h, g = B.solve_grad_logk(logK, dh, Qs, obs)
     assert np.all(np.isfinite(h)) and np.all(np.isfinite(g))
     B.close()
+
+
+@pytest.mark.parametrize("with_last", [0, 1])
+def test_expired_barrier_reports_timeout(lib, with_last):
+    """The grid barrier of the one-launch solves, with a block that never arrives: every thread of the others leaves
+    after the limit of one second."""
+    ms = ctypes.c_double(-1.0)
+    assert lib.dpf_debug_expired_barrier(with_last, ctypes.byref(ms)) == DPF_TIMEOUT
+    assert 900.0 <= ms.value <= 1100.0
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("kind", ["grid", "batch", "parts", "faces"])
+def test_solve_whose_barrier_expires(gpu_lib, lib, kind, precision):
+    """Barriers that wait for a block too many: the one-launch solve gives up after a second, the call is finished by the
+    separate kernels (some hundred launches), and so are the handle's later ones. Both forms solve to 1e-11."""
+    pkg = gpu_lib
+    shapes, mins, maxs, dn, logK, dh, Qs, obs = _case(pkg)
+    if kind == "faces":
+        _, nb, aol, _ = pkg.regulargrid3d(mins[0], maxs[0], shapes[0])
+        n = int(np.prod(shapes[0]))
+        P = pkg.GroundwaterProblem(nb, aol, dn[0], n, general=True, precision=precision, reltol=1e-11)
+        solve = lambda: P.solve_grad_logk(logK[:n], dh[:n], Qs[:n], obs[0])
+    else:
+        k = 1 if kind == "grid" else 2
+        if kind == "parts":     # large enough for one-launch solves in FP64 parts
+            shapes = [(110, 110, 12)] * 2
+            maxs = [tuple(float(n - 1) for n in ns) for ns in shapes]
+            n = int(np.prod(shapes[0]))
+            dn = [np.array([n - 1])] * 2
+            logK, dh, Qs = -9.0 + 0.5 * np.random.default_rng(4).standard_normal(2 * n), np.zeros(2 * n), np.zeros(2 * n)
+            Qs[[0, n]] = 1e-4
+        n = sum(int(np.prod(ns)) for ns in shapes[:k])
+        P = pkg.GroundwaterBatch(shapes[:k], mins[:k], maxs[:k], dn[:k], precision=precision, reltol=1e-11,
+                                 streams=2 if kind == "parts" else 0)
+        solve = lambda: P.solve_grad_logk(logK[:n], dh[:n], Qs[:n], obs[:k])
+
+    def count():
+        l0 = P.launch_count
+        out = solve()
+        return P.launch_count - l0, out
+
+    one, ref = count()
+    assert (one < 100) == (kind != "parts" or precision == "fp64")
+    assert lib.dpf_debug_expire_barriers(P._h, 1) == 0
+    for _ in range(2):
+        many, got = count()
+        assert many > 100
+        assert rel(got[0], ref[0]) < 1e-9 and rel(got[1], ref[1]) < 1e-7
+    P.close()
