@@ -114,6 +114,7 @@ SIGNATURES = {
                                                   ctypes.c_void_p]),
     "dpf_debug_band_order_grids": (ctypes.c_int, [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
     "dpf_debug_check_report": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]),
+    "dpf_debug_check_sites": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int64)]),
 }
 
 _lib = None

@@ -180,6 +180,9 @@ static std::vector<CheckReader> &check_readers() {
     return r;
 }
 void register_check_reader(CheckReader f) { check_readers().push_back(f); }
+#if DPF_CHECKED
+static unsigned g_sites_seen = 0;  // as of the last report
+#endif
 }  // namespace dpf
 
 extern "C" int dpf_debug_check_report(int64_t *violations, int64_t *first) {
@@ -188,10 +191,12 @@ extern "C" int dpf_debug_check_report(int64_t *violations, int64_t *first) {
     bool have = false;
     for (dpf::CheckReader rd : dpf::check_readers()) {
         long long c = 0, f[3] = {0, 0, 0};
-        if (rd(&c, f) != 0) {
+        unsigned seen = 0;
+        if (rd(&c, f, &seen) != 0) {
             dpf::set_global_error("reading the check words failed");
             return DPF_CUDA;
         }
+        dpf::g_sites_seen |= seen;
         if (c > 0 && !have) {
             have = true;
             for (int k = 0; k < 3; k++) f0[k] = f[k];
@@ -205,6 +210,17 @@ extern "C" int dpf_debug_check_report(int64_t *violations, int64_t *first) {
 #else
     (void)violations;
     (void)first;
+    dpf::set_global_error("the library was built without DPF_CHECK");
+    return DPF_UNSUPPORTED;
+#endif
+}
+
+extern "C" int dpf_debug_check_sites(int64_t *sites) {
+#if DPF_CHECKED
+    if (sites) *sites = (int64_t)dpf::g_sites_seen;
+    return DPF_OK;
+#else
+    (void)sites;
     dpf::set_global_error("the library was built without DPF_CHECK");
     return DPF_UNSUPPORTED;
 #endif

@@ -58,13 +58,14 @@ struct GpParams {
 };
 
 // (A x)_i in flux form with the FP64 couplings of the finest level; the diagonal beside it
-__device__ __forceinline__ double gp_flux(const int *rp, const int *ci, const double *v, const double *leak, int i,
+__device__ __forceinline__ double gp_flux(int n, const int *rp, const int *ci, const double *v, const double *leak, int i,
                                           double xi, const double *x, double &diag) {
     const double lk = leak[i];
     double a = lk * xi, d = lk;
     const int e1 = rp[i + 1];
     for (int e = rp[i]; e < e1; e++) {
         const double w = v[e];
+        if (!DPF_INSIDE(CK_ONE_COL, ci[e], 0, n)) continue;
         a += w * (xi - x[ci[e]]);
         d += w;
     }
@@ -106,13 +107,15 @@ __device__ __forceinline__ T gp_resid(const GpLevel<T> &V, const GpRows<T> &R, G
     if constexpr (sizeof(T) == 8) {
         T r = kSmall ? T(0) : fma(-V.dg[i], xi, bi);
         diag = T(0);
-        for (int e = rp[i] + (kSmall ? ln.q : 0); e < e1; e += by) r = fma(v[e], x(e, ci[e]), r);
+        for (int e = rp[i] + (kSmall ? ln.q : 0); e < e1; e += by)
+            if (DPF_INSIDE(CK_ONE_COL, ci[e], 0, V.n)) r = fma(v[e], x(e, ci[e]), r);
         return kSmall ? fma(-V.dg[i], xi, bi) + ln.sum(r) : r;
     } else {
         const T lk = V.leak[i];
         T a = kSmall ? T(0) : lk * xi, d = kSmall ? T(0) : lk;
         for (int e = rp[i] + (kSmall ? ln.q : 0); e < e1; e += by) {
             const T w = v[e];
+            if (!DPF_INSIDE(CK_ONE_COL, ci[e], 0, V.n)) continue;
             a += w * (xi - x(e, ci[e]));
             d += w;
         }
@@ -206,7 +209,7 @@ struct GpSolve {
                         v[k] = V.v[e0 + k];
                         const int j = V.ci[e0 + k];
                         ci[k] = j;
-                        if (nag) aci[k] = V.agg[j];
+                        if (nag) aci[k] = DPF_INSIDE(CK_ONE_COL, j, 0, V.n) ? V.agg[j] : -1;
                     }
                     for (int k = threadIdx.x; k <= m; k += kGpThreads) {
                         rp[k] = V.rp[i0 + k];
@@ -288,7 +291,9 @@ struct GpSolve {
             T r;
             if constexpr (kSmall && FIRST && kFuse) {
                 const T *e = rw[l + 1].xb;
-                auto corr = [&](int a) { return a >= 0 ? P.scale * e[a] : T(0); };
+                auto corr = [&](int a) {
+                    return a >= 0 && DPF_INSIDE(CK_ONE_AGG, a, 0, P.lv[l + 1].n) ? P.scale * e[a] : T(0);
+                };
                 if (!V.dir[i]) xi += corr(V.agg[i]);
                 // coupled cells are free cells
                 r = gp_resid<true>(V, R, ln, i, bi, xi,
@@ -371,7 +376,8 @@ struct GpSolve {
         each_row<kSmall>(i0, i1, lg, [&](int I, GpLane ln, bool store) {
             T a = 0;
             const int k1 = mrp[I + 1];
-            for (int k = mrp[I] + ln.q; k < k1; k += 1 << ln.lg) a += d[mci[k]];
+            for (int k = mrp[I] + ln.q; k < k1; k += 1 << ln.lg)
+                if (DPF_INSIDE(CK_ONE_AGG, mci[k], 0, V.n)) a += d[mci[k]];
             if (kSmall) a = ln.sum(a);
             if (!store) return;
             R.b[I] = a;
@@ -463,7 +469,7 @@ struct GpSolve {
             if (!kFuse || !sm || (l == 0 && deg == 1)) {
                 each_row<false>(rw[l].i0, rw[l].i1, 0, [&](int i, GpLane, bool) {
                     const int a = V.agg[i];
-                    if (a >= 0 && !V.dir[i]) cur[i] += P.scale * e[a];
+                    if (a >= 0 && !V.dir[i] && DPF_INSIDE(CK_ONE_AGG, a, 0, P.lv[l + 1].n)) cur[i] += P.scale * e[a];
                 });
                 if (!step(one)) return false;
             }
@@ -528,7 +534,7 @@ struct GpSolve {
             each([&](int i) {
                 double dg;
                 const double bi = P.b64[i];
-                const double ri = bi - gp_flux(rp, ci, v, P.leak64, i, P.x64[i], P.x64, dg);
+                const double ri = bi - gp_flux(P.lv[0].n, rp, ci, v, P.leak64, i, P.x64[i], P.x64, dg);
                 put_r(i, ri);
                 rr.v += ri * ri;
                 if (!P.dir[i]) bb.v += bi * bi;
@@ -548,7 +554,7 @@ struct GpSolve {
                 Acc<double> a;
                 each([&](int i) {
                     double dg;
-                    const double pi = P.p[i], qi = gp_flux(rp, ci, v, P.leak64, i, pi, P.p, dg);
+                    const double pi = P.p[i], qi = gp_flux(P.lv[0].n, rp, ci, v, P.leak64, i, pi, P.p, dg);
                     P.q[i] = qi;
                     a.v += pi * qi;
                 });
@@ -575,7 +581,7 @@ struct GpSolve {
                 each([&](int i) {
                     double dg;
                     const double xi = P.x64[i], bi = P.b64[i];
-                    const double ri = bi - gp_flux(rp, ci, P.v64, P.leak64, i, xi, P.x64, dg);
+                    const double ri = bi - gp_flux(P.lv[0].n, rp, ci, P.v64, P.leak64, i, xi, P.x64, dg);
                     P.r64[i] = ri;
                     rr.v += ri * ri;
                     if (P.dir[i]) return;  // identity row: in neither
@@ -633,7 +639,9 @@ struct GpSolve {
                         const float2 pi = P.pd[i];
                         float2 v = df_mul(P.leakdf[i], pi);
                         const int e1 = rp[i + 1];
-                        for (int e = rp[i]; e < e1; e++) v = df_add(v, df_mul(P.vdf[e], df_sub(pi, P.pd[ci[e]])));
+                        for (int e = rp[i]; e < e1; e++)
+                            if (DPF_INSIDE(CK_ONE_COL, ci[e], 0, P.lv[0].n))
+                                v = df_add(v, df_mul(P.vdf[e], df_sub(pi, P.pd[ci[e]])));
                         P.qd[i] = v;
                         a = a + Acc<float>::prod(pi.x, v.x);
                     });

@@ -125,6 +125,12 @@ struct Children {
         for (int k = 0; k < 8; k++) {
             const bool in = (!(k & 4) || ox) && (!(k & 2) || oy) && (!(k & 1) || oz);
             const long long i = i0 + (k & 4 ? sx : 0) + (k & 2 ? sy : 0) + (k & 1);
+#if DPF_CHECKED
+            if (in && !DPF_INSIDE(CK_ONE_CHILD, i, Lf.off, Lf.off + Lf.n)) {
+                v[k] = T(0);
+                continue;
+            }
+#endif
             v[k] = in ? x[i] : T(0);
             if (in && !V.dir[i]) on |= 1u << k;
         }

@@ -408,6 +408,10 @@ int dpf_debug_band_order_grids(int nprob, const int32_t *dims, int64_t *perm, in
  * pointer may be NULL). Returns DPF_UNSUPPORTED in a library built without them. */
 int dpf_debug_check_report(int64_t *violations, int64_t *first);
 
+/* No counterpart in the reference. The checks such a library had evaluated by the last dpf_debug_check_report: bit k of
+ * *sites (may be NULL) for site code k. DPF_UNSUPPORTED in a library built without them. */
+int dpf_debug_check_sites(int64_t *sites);
+
 #ifdef __cplusplus
 }
 #endif
