@@ -1466,9 +1466,13 @@ void GeneralSolver::solve(const double *b, double *x) {
     if (opt.solver == DPF_SOLVER_CHOLESKY && direct_solve(b, x)) return;
     NvtxRange range("CG + AMG solve (CSR)");
     const double tol2 = opt.reltol * opt.reltol;
-    // one launch, except where per-kernel profiles or host-driven loops are asked for
+    // one launch, except where per-kernel profiles or host-driven loops are asked for, and on mixed handles of more
+    // than 5 Mi cells: there the gathers come from DRAM, and one block of 1024 threads per SM has half the loads in
+    // flight that the separate kernels have. One launch -> separate, mixed: fracture networks of 2M cells 80.5 -> 108 ms,
+    // 5.1M 232 -> 231, 11M 544 -> 464; grids as face lists of 2M 26.9 -> 30.8, 4.1M 50.1 -> 49.9, 6.4M 86.9 -> 77.7, shuffled
+    // 4.1M 77.4 -> 84.4, 6.4M 122 -> 125. FP64, whose steps are bound by its arithmetic: 11M 718 -> 1038 ms.
     bool done = false;
-    if (persist_blocks && opt.use_graphs && !prof_on) {
+    if (persist_blocks && opt.use_graphs && !prof_on && !(mixed && N > 5 << 20)) {
         if (mixed) solve_persistent<float>(b, x, tol2);
         else solve_persistent<double>(b, x, tol2);
         from_dev(h_state, d_state, sizeof(CgState));

@@ -133,6 +133,38 @@ def test_face_lists(gpu_lib, orc, kind, degree, precision):
         assert rel(g, w) < 1e-6
 
 
+def _launches(pkg, n, nb, dn, **opt):
+    rng = np.random.default_rng(5)
+    P = pkg.GroundwaterProblem(nb, rng.uniform(0.5, 2.0, len(nb)), dn, N=n, general=True, **opt)
+    Qs = np.zeros(n)
+    Qs[np.setdiff1d(np.arange(min(n, 1000)), dn)[3]] = 1e-4
+    l0 = P.launch_count
+    P.forward(np.exp(-9.0 + rng.standard_normal(len(nb))), np.zeros(n), Qs)
+    launches = P.launch_count - l0
+    P.close()
+    return launches
+
+
+@pytest.mark.parametrize("precision", ["fp64", "mixed"])
+@pytest.mark.parametrize("kind", ["grid42", "grid529", "grid3570", "tree", "pairs"])
+def test_face_lists_take_one_launch(gpu_lib, kind, precision):
+    """The meshes of the tests around this one are solved by the one-launch kernel."""
+    n, nb, dn = _mesh(kind)
+    one, many = (_launches(gpu_lib, n, nb, dn, precision=precision, reltol=1e-12, use_graphs=g) for g in (1, 0))
+    assert one < many and one < 60
+
+
+def test_large_mixed_face_list_takes_separate_launches(gpu_lib):
+    """Above 5 Mi cells the separate kernels are the faster ones: the same launches as with the loop on the host."""
+    nx, ny = 2300, 2290
+    i = np.arange(nx * ny).reshape(nx, ny)
+    nb = np.concatenate([np.stack([i[:-1].ravel(), i[1:].ravel()], 1), np.stack([i[:, :-1].ravel(), i[:, 1:].ravel()], 1)])
+    opt = {"precision": "mixed", "maxiter": 2, "max_outer": 1}
+    assert i.size > 5 << 20
+    with pytest.warns(RuntimeWarning, match="did not reach its tolerance"):
+        assert len({_launches(gpu_lib, i.size, nb, np.array([0, i.size - 1]), use_graphs=g, **opt) for g in (1, 0)}) == 1
+
+
 @pytest.mark.parametrize("precision", ["fp64", "mixed"])
 @pytest.mark.parametrize("degree", [1, 2, 3])
 def test_face_lists_levels_of_both_kinds(gpu_lib, degree, precision):
