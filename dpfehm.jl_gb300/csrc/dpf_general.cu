@@ -1354,11 +1354,11 @@ __global__ void kg_front_fill(int n, GOp<double> A, const int *__restrict__ iper
 // As StructBatch::choose_direct.
 void GeneralSolver::choose_direct() {
     if (opt.solver != DPF_SOLVER_CHOLESKY || direct_tried) return;
-    direct_tried = true;
     size_t free_b = 0, total_b = 0;
     GCK(cudaMemGetInfo(&free_b, &total_b));
-    if (N >= kFrontMaxCells || !direct_fits(N, band_order_rcm(N, hrp_, hci_).w, free_b / 2)) return;
-    fronts = make_fronts(dissect_graph((int)N, hrp_, hci_), hrp_, hci_, free_b / 10 * 9, stream);
+    if (N < kFrontMaxCells && direct_fits(N, band_order_rcm(N, hrp_, hci_).w, free_b / 2))
+        fronts = make_fronts(dissect_graph((int)N, hrp_, hci_), hrp_, hci_, free_b / 10 * 9, stream);
+    direct_tried = true;
 }
 
 bool GeneralSolver::direct_solve(const double *b, double *x) {

@@ -3080,7 +3080,6 @@ void StructBatch::apply(const double *x, double *y) {
 // assembly, which then leaves out the multigrid hierarchy that only the iterative solver needs.
 void StructBatch::choose_direct() {
     if (opt.solver != DPF_SOLVER_CHOLESKY || direct_tried) return;
-    direct_tried = true;
     Level &L0 = lv[0];
     std::vector<std::array<int, 3>> dims;
     std::vector<long long> off;
@@ -3091,10 +3090,12 @@ void StructBatch::choose_direct() {
     }
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
-    if (N >= kFrontMaxCells || !direct_fits(N, band_order_regular(dims, off).w, free_b / 2)) return;
-    std::vector<int> rp, ci;
-    regular_graph(dims, off, rp, ci);
-    fronts = make_fronts(dissect_regular(dims, off), rp, ci, free_b / 10 * 9, stream);
+    if (N < kFrontMaxCells && direct_fits(N, band_order_regular(dims, off).w, free_b / 2)) {
+        std::vector<int> rp, ci;
+        regular_graph(dims, off, rp, ci);
+        fronts = make_fronts(dissect_regular(dims, off), rp, ci, free_b / 10 * 9, stream);
+    }
+    direct_tried = true;  // behind the allocations: where one fails, the next assembly tries again
 }
 
 bool StructBatch::direct_solve(const double *b, double *x) {

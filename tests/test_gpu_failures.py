@@ -138,6 +138,38 @@ def test_general_path_allocation_failure(gpu_lib, lib):
         assert _stats(lib)[1] == live0, k
 
 
+@pytest.mark.parametrize("general", [False, True])
+def test_each_direct_solve_allocation_failure(gpu_lib, lib, general):
+    """A first direct solve whose k-th allocation fails reports DPF_OOM; the next one on the same handle is direct."""
+    pkg = gpu_lib
+    _, nb, aol, _ = pkg.regulargrid3d((0.0, 0.0, 0.0), (9.0, 7.0, 3.0), (10, 8, 4))
+    N = 320
+    Ks = np.exp(np.random.default_rng(5).normal(-9, 0.5, len(nb)))
+    Qs = np.zeros(N)
+    Qs[0] = 1e-4
+    make = lambda: pkg.GroundwaterProblem(nb, aol, [N - 1], N, general=general, solver="cholesky")
+    live0 = _stats(lib)[1]
+    P = make()
+    m0 = _stats(lib)[0]
+    h_ref = P.forward(Ks, np.zeros(N), Qs)
+    assert P.stats["iterations"] == 0
+    count = _stats(lib)[0] - m0
+    P.close()
+    assert count > 10
+    for k in range(count):
+        P = make()
+        lib.dpf_debug_fail_alloc(k)
+        with pytest.raises(pkg.DPFError) as ei:
+            P.forward(Ks, np.zeros(N), Qs)
+        assert ei.value.code == DPF_OOM, (k, str(ei.value))
+        lib.dpf_debug_fail_alloc(-1)
+        h = P.forward(Ks, np.zeros(N), Qs)
+        assert P.stats["iterations"] == 0, k
+        assert rel(h, h_ref) < 1e-12, k
+        P.close()
+        assert _stats(lib)[1] == live0, k
+
+
 def test_expired_wait_reports_timeout(gpu_lib, lib):
     pkg = gpu_lib
     ms = ctypes.c_double(-1.0)
