@@ -113,6 +113,8 @@ SIGNATURES = {
     "dpf_debug_band_order_graph": (ctypes.c_int, [ctypes.c_int64, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p,
                                                   ctypes.c_void_p]),
     "dpf_debug_band_order_grids": (ctypes.c_int, [ctypes.c_int, ctypes.c_void_p, ctypes.c_void_p, ctypes.c_void_p]),
+    "dpf_debug_direct_fronts": (ctypes.c_int, [_i64, _vp, _vp, _i64, _ip, _i64p, _f64p]),
+    "dpf_debug_direct_memory": (ctypes.c_int, [_vp, _i64]),
     "dpf_debug_check_report": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int64), ctypes.POINTER(ctypes.c_int64)]),
     "dpf_debug_check_sites": (ctypes.c_int, [ctypes.POINTER(ctypes.c_int64)]),
 }

@@ -236,6 +236,14 @@ extern "C" int dpf_debug_expire_barriers(dpf_problem *P, int on) {
     return DPF_OK;
 }
 
+extern "C" int dpf_debug_direct_memory(dpf_problem *P, int64_t bytes) {
+    if (!P || bytes < 0) return DPF_BAD_INPUT;
+    for (dpf_problem *Q : P->parts) dpf_debug_direct_memory(Q, bytes);
+    if (P->sb) P->sb->direct_memory = (size_t)bytes;
+    if (P->gs) P->gs->direct_memory = (size_t)bytes;
+    return DPF_OK;
+}
+
 extern "C" void dpf_debug_alloc_stats(int64_t *made, int64_t *live) {
     if (made) *made = dpf::g_made.load();
     if (live) *live = dpf::g_live.load();

@@ -13,6 +13,7 @@
 #include <string>
 
 #include "dpf_direct.h"
+#include "dpf_front.h"
 #include "dpf_grid.cuh"
 #include "dpf_means.cuh"
 #include "dpf_plane.cuh"
@@ -191,6 +192,36 @@ extern "C" int dpf_debug_band_order_graph(int64_t n, const int32_t *rp, const in
         const dpf::BandOrder o = dpf::band_order_rcm((long long)n, r, c);
         for (int64_t k = 0; k < n; k++) perm[k] = o.perm[k];
         *w = o.w;
+    } catch (const std::bad_alloc &) {
+        return DPF_OOM;
+    }
+    return DPF_OK;
+}
+
+extern "C" int dpf_debug_direct_fronts(int64_t n, const int32_t *rp, const int32_t *ci, int64_t free_bytes, int *form,
+                                       int64_t *max_rows, double *bytes) {
+    if (n < 1 || n >= dpf::kFrontMaxCells || !rp || !form || !max_rows || !bytes || free_bytes < 0) return DPF_BAD_INPUT;
+    if (rp[0] != 0) return DPF_BAD_INPUT;
+    for (int64_t i = 0; i < n; i++)
+        if (rp[i + 1] < rp[i]) return DPF_BAD_INPUT;
+    if (rp[n] > 0 && !ci) return DPF_BAD_INPUT;
+    for (int32_t e = 0; e < rp[n]; e++)
+        if (ci[e] < 0 || ci[e] >= n) return DPF_BAD_INPUT;
+    try {
+        std::vector<int> r(rp, rp + n + 1), c(ci, ci + rp[n]);
+        const dpf::BandOrder band = dpf::band_order_rcm((long long)n, r, c);
+        *form = 0;
+        *max_rows = 0;
+        *bytes = 0.0;
+        if (!dpf::direct_fits((long long)n, band.w, (size_t)free_bytes / 2)) return DPF_OK;
+        dpf::Dissection d = dpf::dissect_graph((int)n, r, c);
+        const size_t nodes = d.k.size();
+        const std::vector<int> perm = d.perm;
+        dpf::FrontTree t;
+        const bool fits = dpf::choose_fronts(d, band, r, c, (size_t)free_bytes, t);
+        *form = !fits ? -1 : d.k.size() == nodes && d.perm == perm ? 1 : 2;
+        *max_rows = t.max_m;
+        *bytes = t.bytes();
     } catch (const std::bad_alloc &) {
         return DPF_OOM;
     }

@@ -633,6 +633,17 @@ Dissection dissect_graph(int n, const std::vector<int> &rp, const std::vector<in
     return B.d;
 }
 
+Dissection dissect_band(const BandOrder &o) {
+    Builder B;
+    const int n = (int)o.perm.size(), nodes = blocks_of(n, kBandBlock);
+    for (int s = 0; s < nodes; s++) {
+        const int a = s * kBandBlock, b = std::min(n, a + kBandBlock);
+        B.add(std::vector<int>(o.perm.begin() + a, o.perm.begin() + b), nodes - 1 - s,
+              s ? std::vector<int>{s - 1} : std::vector<int>{});
+    }
+    return B.d;
+}
+
 void regular_graph(const std::vector<std::array<int, 3>> &dims, const std::vector<long long> &off,
                    std::vector<int> &rp, std::vector<int> &ci) {
     long long n = 0;
@@ -855,10 +866,17 @@ FrontSolver::FrontSolver(const Dissection &d, const FrontTree &t, cudaStream_t s
     }
 }
 
-std::unique_ptr<FrontSolver> make_fronts(const Dissection &d, const std::vector<int> &rp, const std::vector<int> &ci,
-                                         size_t max_bytes, cudaStream_t stream) {
+bool choose_fronts(Dissection &d, const BandOrder &band, const std::vector<int> &rp, const std::vector<int> &ci,
+                   size_t free_bytes, FrontTree &t) {
+    if (build_fronts(d, rp, ci, 0.5 * (double)free_bytes, t) && t.max_m <= FrontSolver::kMaxM) return true;
+    d = dissect_band(band);
+    return build_fronts(d, rp, ci, 0.9 * (double)free_bytes, t) && t.max_m <= FrontSolver::kMaxM;
+}
+
+std::unique_ptr<FrontSolver> make_fronts(Dissection d, const BandOrder &band, const std::vector<int> &rp,
+                                         const std::vector<int> &ci, size_t free_bytes, cudaStream_t stream) {
     FrontTree t;
-    if (!build_fronts(d, rp, ci, (double)max_bytes, t) || t.max_m > FrontSolver::kMaxM) return nullptr;
+    if (!choose_fronts(d, band, rp, ci, free_bytes, t)) return nullptr;
     return std::unique_ptr<FrontSolver>(new FrontSolver(d, t, stream));
 }
 

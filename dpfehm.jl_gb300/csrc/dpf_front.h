@@ -20,6 +20,8 @@
 #include <memory>
 #include <vector>
 
+#include "dpf_direct.h"
+
 namespace dpf {
 
 constexpr long long kFrontMaxCells = 300000000;  // 32-bit cell and coupling numbers
@@ -42,6 +44,10 @@ struct Dissection {
 };
 Dissection dissect_regular(const std::vector<std::array<int, 3>> &dims, const std::vector<long long> &off);
 Dissection dissect_graph(int n, const std::vector<int> &rp, const std::vector<int> &ci);
+// A band order cut into runs of kBandBlock rows, each the parent of the one before: its fronts have at most
+// kBandBlock + w rows, whatever the graph.
+constexpr int kBandBlock = 64;
+Dissection dissect_band(const BandOrder &o);
 
 // Fronts of a dissection for the couplings of a symmetric graph (CSR, original numbering).
 struct FrontTree {
@@ -126,8 +132,13 @@ private:
     long long panel_size = 0;
 };
 
-// The fronts of a dissection, or null where they do not fit max_bytes.
-std::unique_ptr<FrontSolver> make_fronts(const Dissection &d, const std::vector<int> &rp, const std::vector<int> &ci,
-                                         size_t max_bytes, cudaStream_t stream);
+// The fronts for a system that direct_fits accepted: those of its nested dissection within half the free
+// memory, otherwise those of its band order within nine tenths of it. A dissection's fronts take less than the band
+// but where the graph has no small separators: 8000 cells in two sets with couplings between the sets only want
+// 18.8 GB, their band 0.5. False where neither fits.
+bool choose_fronts(Dissection &d, const BandOrder &band, const std::vector<int> &rp, const std::vector<int> &ci,
+                   size_t free_bytes, FrontTree &t);
+std::unique_ptr<FrontSolver> make_fronts(Dissection d, const BandOrder &band, const std::vector<int> &rp,
+                                         const std::vector<int> &ci, size_t free_bytes, cudaStream_t stream);
 
 }  // namespace dpf

@@ -1356,8 +1356,10 @@ void GeneralSolver::choose_direct() {
     if (opt.solver != DPF_SOLVER_CHOLESKY || direct_tried) return;
     size_t free_b = 0, total_b = 0;
     GCK(cudaMemGetInfo(&free_b, &total_b));
-    if (N < kFrontMaxCells && direct_fits(N, band_order_rcm(N, hrp_, hci_).w, free_b / 2))
-        fronts = make_fronts(dissect_graph((int)N, hrp_, hci_), hrp_, hci_, free_b / 10 * 9, stream);
+    if (direct_memory) free_b = direct_memory;
+    const BandOrder band = band_order_rcm(N, hrp_, hci_);
+    if (N < kFrontMaxCells && direct_fits(N, band.w, free_b / 2))
+        fronts = make_fronts(dissect_graph((int)N, hrp_, hci_), band, hrp_, hci_, free_b, stream);
     direct_tried = true;
 }
 

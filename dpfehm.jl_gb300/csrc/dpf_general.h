@@ -78,6 +78,7 @@ public:
     void profile(bool on);
     int profile_report(int cap, const char **names, long long *counts, double *ms, long long *cells);
     std::string last_message;
+    size_t direct_memory = 0;    // test hook: the free memory that the direct solver sees (0: the device's)
     bool barrier_short = false;  // test hook: one arrival too few at the one-launch solve's barriers
 
 private:

@@ -3090,10 +3090,12 @@ void StructBatch::choose_direct() {
     }
     size_t free_b = 0, total_b = 0;
     CK(cudaMemGetInfo(&free_b, &total_b));
-    if (N < kFrontMaxCells && direct_fits(N, band_order_regular(dims, off).w, free_b / 2)) {
+    if (direct_memory) free_b = direct_memory;
+    const BandOrder band = band_order_regular(dims, off);
+    if (N < kFrontMaxCells && direct_fits(N, band.w, free_b / 2)) {
         std::vector<int> rp, ci;
         regular_graph(dims, off, rp, ci);
-        fronts = make_fronts(dissect_regular(dims, off), rp, ci, free_b / 10 * 9, stream);
+        fronts = make_fronts(dissect_regular(dims, off), band, rp, ci, free_b, stream);
     }
     direct_tried = true;  // behind the allocations: where one fails, the next assembly tries again
 }

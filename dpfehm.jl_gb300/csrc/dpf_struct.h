@@ -169,6 +169,7 @@ public:
     double2 *d_ppart = nullptr;      // its reduction slots
     int persist_blocks = 0;          // blocks of the cooperative launch (0: not available)
     bool barrier_short = false;      // test hook: one arrival too few
+    size_t direct_memory = 0;        // test hook: the free memory that the direct solver sees (0: the device's)
     cudaGraphExec_t loop_graph(int kind, void *x);
     void run_loop(int kind, void *x);
     int read_count(int which);

@@ -400,6 +400,16 @@ int dpf_debug_pow64(int64_t n, const double *x, const double *y, double *p, doub
 int dpf_debug_band_order_graph(int64_t n, const int32_t *rp, const int32_t *ci, int64_t *perm, int64_t *w);
 int dpf_debug_band_order_grids(int nprob, const int32_t *dims, int64_t *perm, int64_t *w);
 
+/* No counterpart in the reference. What the direct solver takes for such a graph with free_bytes of free device memory
+ * (host code): *form 0: refused by its band, 1: the fronts of a nested dissection, 2: those of the band order, -1: neither
+ * fits; with the rows of the largest front and their memory. */
+int dpf_debug_direct_fronts(int64_t n, const int32_t *rp, const int32_t *ci, int64_t free_bytes, int *form,
+                            int64_t *max_rows, double *bytes);
+
+/* No counterpart in the reference. The free device memory that a handle's direct solver is to reckon with (0: the
+ * device's); before its first solve. */
+int dpf_debug_direct_memory(dpf_problem *p, int64_t bytes);
+
 /* No counterpart in the reference. In a library built with DPF_CHECK defined
  * (device-side bounds and alignment checks on cell decodes, stencil neighbours,
  * aggregates, staged copies and CSR columns; a violating access is clamped or

@@ -58,3 +58,26 @@ def test_mesh_fronts(gpu_lib, orc, kind):
     assert rel(got[0], want[0]) < 1e-11
     for g, w in zip(got[1:], want[1:]):
         assert rel(g, w) < 1e-9
+
+
+def test_band_fronts(gpu_lib, orc):
+    """A graph without small separators, with the memory for its band but not for its dissection: the fronts of the band
+    order, 64 rows each with a remainder. Tolerances as above."""
+    from test_direct_fronts import two_sets
+    n, nb = two_sets(205, 0.3)
+    rng = np.random.default_rng(8)
+    aol, Ks = rng.uniform(0.5, 2.0, len(nb)), np.exp(-9.0 + rng.standard_normal(len(nb)))
+    dn = np.array([3, 250])
+    dh, Qs, delta = np.zeros(n), np.zeros(n), rng.standard_normal(n)
+    dh[dn] = rng.uniform(0, 1, len(dn))
+    Qs[[7, 100, 300]] = [1e-4, 5e-5, -2e-5]
+    P = gpu_lib.GroundwaterProblem(nb, aol, dn, N=n, general=True, solver="cholesky")
+    assert gpu_lib.load().dpf_debug_direct_memory(P._h, 3300000) == 0
+    O = orc.Problem(n, nb, aol, dn)
+    want = (O.steady(Ks, dh, Qs, reltol=1e-14),) + tuple(O.adjoint(dh, delta, reltol=1e-14))
+    for _ in range(2):
+        got = (P.forward(Ks, dh, Qs),) + tuple(P.adjoint(delta))
+        assert P.stats["iterations"] == 0 and P.stats["relres"] < 1e-12
+        assert rel(got[0], want[0]) < 1e-11
+        for g, w in zip(got[1:], want[1:]):
+            assert rel(g, w) < 1e-9
