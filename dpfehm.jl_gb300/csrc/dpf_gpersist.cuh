@@ -7,8 +7,8 @@
 // The finest level's steps are near the memory's rate (9..17 us each: gathers through the column indices);
 // a step on a small level takes 3..4 us, of which a barrier is 1.3. Those steps are bound by trips to L2:
 // a block keeps its rows of the small levels in shared memory, 2 to 8 lanes (FP64: 4) share a row, and the ranges of
-// a block's rows are worked out once (they cost two integer divisions per step). Together 51.3 -> 45.6 ms
-// and 34.3 -> 31.0 ms.
+// a block's rows are worked out once (they cost two integer divisions per step). Together 51.3 -> 44.3 ms
+// and 34.3 -> 31.3 ms.
 //
 // Per level the rows are cut into equal contiguous shares of whole groups of 32, one per block; the levels
 // of a few hundred cells run in one block. The first smoothing pass reads u = b D^-1, stored by the pass

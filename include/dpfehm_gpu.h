@@ -89,7 +89,9 @@ typedef struct dpf_options {
     int max_coarse;      /* coarsen until a level has at most this many cells (default 64, <= 64) */
     int max_outer;       /* MIXED: cap on rounds, each restarted from the true FP64 residual (default 6) */
     int use_graphs;      /* default 1: a solve runs as one cooperative launch (face lists, FP64 grids and
-                            small MIXED grids) or as a CUDA graph (large MIXED grids); 0: as separate
+                            small MIXED grids), or, where that is the slower form, as a CUDA graph (large MIXED
+                            grids, batches of very uneven sizes or in concurrent parts) or separate launches
+                            (MIXED face lists above 5 Mi cells); 0: as separate
                             launches with a convergence check on the host */
     int check_every;     /* separate launches (use_graphs = 0): convergence is read back every this many
                             iterations (default 1); the general path reads only every eighth until two
