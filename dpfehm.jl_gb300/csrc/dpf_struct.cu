@@ -304,7 +304,11 @@ __device__ __forceinline__ T cell_cheb_step(const LevelDesc &L, const Cell &c, c
                                             const T *__restrict__ b, const T *__restrict__ xin,
                                             T *__restrict__ xout, T *__restrict__ d, T c1, T c2, T &bi) {
     T xi = ldv<CG>(xin, c.i), dg;
-    const T ri = resid7(L, c, C, [&] { return bi = ldv<CG>(b, c.i); }, xi,
+    if constexpr (sizeof(T) == 8) bi = ldv<CG>(b, c.i);
+    const T ri = resid7(L, c, C, [&] {
+                            if constexpr (sizeof(T) == 4) bi = ldv<CG>(b, c.i);
+                            return bi;
+                        }, xi,
                         [&](long long j, int, int, int) { return ldv<CG>(xin, j); }, dg);
     T dn, xo;
     if constexpr (sizeof(T) == 8) {
@@ -335,8 +339,12 @@ __device__ __forceinline__ T cell_restrict(const LevelDesc &L, const Cell &cc, c
                 c.ix = fx; c.iy = fy; c.iz = fz;
                 c.i = L.off + fx * fsx + fy * fsy + fz;
                 T xi = ldv<CG>(x, c.i), dg;
-                acc += resid7(L, c, C, [&] { return ldv<CG>(b, c.i); }, xi,
-                              [&](long long j, int, int, int) { return ldv<CG>(x, j); }, dg);
+                T bi;
+                if constexpr (sizeof(T) == 8) bi = ldv<CG>(b, c.i);
+                acc += resid7(L, c, C, [&] {
+                                  if constexpr (sizeof(T) == 4) bi = ldv<CG>(b, c.i);
+                                  return bi;
+                              }, xi, [&](long long j, int, int, int) { return ldv<CG>(x, j); }, dg);
             }
     return acc;
 }
